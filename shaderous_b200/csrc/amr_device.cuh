@@ -14,7 +14,7 @@
 #include <cstdint>
 
 #include "amr_kernels.h"
-#include "hydro_cell.cuh"
+#include "block_math.cuh"
 #include "hydro_math.cuh"
 
 namespace shz {

@@ -98,7 +98,7 @@ __device__ __noinline__ void predict_texel(const KParams& P, const int* __restri
     lp[a] += 1;
     load_w6<DIM>(w1, w2, slot, lm, m);
     load_w6<DIM>(w1, w2, slot, lp, p);
-    axis_edges<R, ISEN>(m, m, c, p, p, P.inv_gamma, sua[a], sda[a]);
+    axis_edges<R, ISEN>(m, c, p, P.inv_gamma, sua[a], sda[a]);
     conv += p[1 + a] - m[1 + a];
     jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
   }
@@ -114,7 +114,7 @@ __device__ __noinline__ void predict_texel(const KParams& P, const int* __restri
     load_w7<DIM>(w1, w2, slot, l0, g);
     load_w6<DIM>(w1, w2, slot, lm, m);
     load_w6<DIM>(w1, w2, slot, lp, p);
-    axis_edges<R, ISEN>(m, m, g, p, p, P.inv_gamma, su, sd);
+    axis_edges<R, ISEN>(m, g, p, P.inv_gamma, su, sd);
   } else {
 #pragma unroll
     for (int v = 0; v < 6; v++) {
@@ -460,20 +460,20 @@ __global__ void __maxnreg__(80)
         float m[7], p[7];
         read_w7(pj, lx - 1, ly, m);
         read_w7(pj, lx + 1, ly, p);
-        axis_edges<R, ISEN>(m, m, c, p, p, P.inv_gamma, su[0], sd[0]);
+        axis_edges<R, ISEN>(m, c, p, P.inv_gamma, su[0], sd[0]);
         conv += p[1] - m[1];
         jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
         if constexpr (DIM >= 2) {
           read_w7(pj, lx, ly - 1, m);
           read_w7(pj, lx, ly + 1, p);
-          axis_edges<R, ISEN>(m, m, c, p, p, P.inv_gamma, su[1], sd[1]);
+          axis_edges<R, ISEN>(m, c, p, P.inv_gamma, su[1], sd[1]);
           conv += p[2] - m[2];
           jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
         }
         if constexpr (DIM == 3) {
           read_w7(ring(j - 1), lx, ly, m);
           read_w7(ring(j + 1), lx, ly, p);
-          axis_edges<R, ISEN>(m, m, c, p, p, P.inv_gamma, su[2], sd[2]);
+          axis_edges<R, ISEN>(m, c, p, P.inv_gamma, su[2], sd[2]);
           conv += p[3] - m[3];
           jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
         }

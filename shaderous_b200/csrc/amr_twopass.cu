@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(NT) amr_predict(const KParams* __restrict__ gp
         lp[a] += 1;
         load_w<DIM>(w1, w2, src, lm, m);
         load_w<DIM>(w1, w2, src, lp, p);
-        axis_edges<R, ISEN>(m, m, c, p, p, P.inv_gamma, su[a], sd[a]);
+        axis_edges<R, ISEN>(m, c, p, P.inv_gamma, su[a], sd[a]);
         conv += p[1 + a] - m[1 + a];
         jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
       }
@@ -90,8 +90,8 @@ __device__ __forceinline__ void face_flux(const KParams& P, const float4* __rest
   load_w<DIM>(w1, w2, slot, b, wb);
   load_w<DIM>(w1, w2, slot, bp, wbp);
   float su[6], sd[6], tu[6], td[6];
-  axis_edges<R, ISEN>(wm, wm, wa, wb, wb, P.inv_gamma, su, sd);   // cell a: toward its upper face
-  axis_edges<R, ISEN>(wa, wa, wb, wbp, wbp, P.inv_gamma, tu, td);  // cell b: from its lower face
+  axis_edges<R, ISEN>(wm, wa, wb, P.inv_gamma, su, sd);   // cell a: toward its upper face
+  axis_edges<R, ISEN>(wa, wb, wbp, P.inv_gamma, tu, td);  // cell b: from its lower face
   Pred pa, pb;
   {
     const size_t o = (size_t)slot * BG<DIM>::PN + ptex<DIM>(a);

@@ -33,13 +33,15 @@
 #include <cstdint>
 #include <cstdio>
 
-#include "hydro_cell.cuh"
 #include "hydro_math.cuh"
 #include "diag_ext.cuh"
 #include "sweep.h"
+#include "sweep_math.cuh"
 #include "tma.cuh"
 
 namespace shz {
+
+using namespace uni;
 
 template <int DIM, int RECON>
 struct Geo {
@@ -366,9 +368,10 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
         read_w<DIM, RECON>(sWj, wx, wy, a0);
         read_w<DIM, RECON>(ringk(1), wx, wy, b1);
 #pragma unroll
-        for (int v = 0; v < 6; v++) {
-          zs_m[v] = ppm_slope(c2[v], c1[v], a0[v]);
-          zs_0[v] = ppm_slope(c1[v], a0[v], b1[v]);
+        for (int i = 0; i < 3; i++) {
+          const float2 d = sub2(pair(a0, i), pair(c1, i));
+          put2(zs_m, i, ppm_slope2(sub2(pair(c1, i), pair(c2, i)), d));
+          put2(zs_0, i, ppm_slope2(d, sub2(pair(b1, i), pair(a0, i))));
         }
         zs_ready = true;
       }
@@ -379,11 +382,15 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
       float p2v[6];
       read_w<DIM, RECON>(ringk(2), wx, wy, p2v);
 #pragma unroll
-      for (int v = 0; v < 6; v++) {
-        const float zp = ppm_slope(c[v], p[v], p2v[v]);
-        ppm_incs_d(m[v], c[v], p[v], zs_m[v], zs_0[v], zp, su_z[v], sd_z[v]);
-        zs_m[v] = zs_0[v];
-        zs_0[v] = zp;
+      for (int i = 0; i < 3; i++) {
+        const float2 cc = pair(c, i), pp = pair(p, i), dr = sub2(pp, cc);
+        const float2 sp = ppm_slope2(dr, sub2(pair(p2v, i), pp)), s0 = pair(zs_0, i);
+        float2 u, d;
+        ppm_edges2(sub2(cc, pair(m, i)), dr, pair(zs_m, i), s0, sp, u, d);
+        put2(su_z, i, u);
+        put2(sd_z, i, d);
+        put2(zs_m, i, s0);
+        put2(zs_0, i, sp);
       }
     };
 
@@ -396,6 +403,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
         float c[7], m[7], p[7], m2[7], p2[7], su[6], sd[6];
         read_w<DIM, RECON>(sWj, wx, wy, c);
         with_cs(c, P);
+        const CellInv ci = cell_inv(c);
         read_w<DIM, RECON>(ringk(-1), wx, wy, m);
         read_w<DIM, RECON>(ringk(1), wx, wy, p);
         if constexpr (ZCARRY) {
@@ -403,7 +411,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
           (void)p2;
           z_edges(m, c, p, su, sd);
         } else {
-          axis_edges<RECON, ISEN>(m2, m, c, p, p2, P.inv_gamma, su, sd);
+          axis_edges<RECON, ISEN>(m2, m, c, p, p2, ci, P.inv_gamma, su, sd);
         }
         if (zg_lo) {
 #pragma unroll
@@ -420,7 +428,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
           face_state(g, sd, -1.f, zlo);
           riemann<2>(zhi_prev, zlo, P, Fz, flagged_prev);
 #pragma unroll
-          for (int v = 0; v < 8; v++) acc[v] -= Fz[v];
+          for (int i = 0; i < 4; i++) put2(acc, i, sub2(pair(acc, i), pair(Fz, i)));
           const size_t o = ((size_t)(j - 1) * ny + gy) * nx + gx;
           float4 na, nb;
           update_cell(__ldg(u1 + o), __ldg(u2 + o), acc, ph_prev, dtdx, P, na, nb);
@@ -436,6 +444,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
     float c[7];
     read_w<DIM, RECON>(sWj, wx, wy, c);
     with_cs(c, P);
+    const CellInv ci = cell_inv(c);
     float su[DIM][6], sd[DIM][6];
     float conv = 0.f, jump = -INFINITY;
     {
@@ -446,7 +455,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
         read_w<DIM, RECON>(sWj, wx - 2, wy, m2);
         read_w<DIM, RECON>(sWj, wx + 2, wy, p2);
       }
-      axis_edges<RECON, ISEN>(m2, m, c, p, p2, P.inv_gamma, su[0], sd[0]);
+      axis_edges<RECON, ISEN>(m2, m, c, p, p2, ci, P.inv_gamma, su[0], sd[0]);
       conv += p[1] - m[1];
       jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
       if constexpr (DIM >= 2) {
@@ -456,7 +465,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
           read_w<DIM, RECON>(sWj, wx, wy - 2, m2);
           read_w<DIM, RECON>(sWj, wx, wy + 2, p2);
         }
-        axis_edges<RECON, ISEN>(m2, m, c, p, p2, P.inv_gamma, su[1], sd[1]);
+        axis_edges<RECON, ISEN>(m2, m, c, p, p2, ci, P.inv_gamma, su[1], sd[1]);
         conv += p[2] - m[2];
         jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
       }
@@ -466,7 +475,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
         if constexpr (ZCARRY) {
           z_edges(m, c, p, su[2], sd[2]);
         } else {
-          axis_edges<RECON, ISEN>(m2, m, c, p, p2, P.inv_gamma, su[2], sd[2]);
+          axis_edges<RECON, ISEN>(m2, m, c, p, p2, ci, P.inv_gamma, su[2], sd[2]);
         }
         conv += p[3] - m[3];
         jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
@@ -474,7 +483,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
     }
     (void)wo;
     Pred pr;
-    hancock<DIM>(c, conv, jump, su, sd, h, P, pr);
+    hancock<DIM>(c, ci.r, conv, jump, su, sd, h, P, pr);
 
     const bool tile_plane = j >= z0 && j < z1;
     // 3. ghosts across outflow / reflecting x/y boundaries take the inner cell's half step.
@@ -556,7 +565,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
       if constexpr (DIM == 3) {
         if (j - 1 >= z0) {
 #pragma unroll
-          for (int v = 0; v < 8; v++) acc[v] -= Fz[v];
+          for (int i = 0; i < 4; i++) put2(acc, i, sub2(pair(acc, i), pair(Fz, i)));
           const size_t o = ((size_t)(j - 1) * ny + gy) * nx + gx;
           float4 na, nb;
           update_cell(__ldg(u1 + o), __ldg(u2 + o), acc, ph_prev, dtdx, P, na, nb);
@@ -574,15 +583,11 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
           unpack8(sFlux[2 * PN + tid + PX], sFlux[3 * PN + tid + PX], yu);
         }
 #pragma unroll
-        for (int v = 0; v < 8; v++) {
-          float a = xl[v];
-          a -= xu[v];
-          if constexpr (DIM >= 2) {
-            a += yl[v];
-            a -= yu[v];
-          }
-          if constexpr (DIM == 3) a += Fz[v];
-          acc[v] = a;
+        for (int i = 0; i < 4; i++) {
+          float2 a = sub2(pair(xl, i), pair(xu, i));
+          if constexpr (DIM >= 2) a = sub2(add2(a, pair(yl, i)), pair(yu, i));
+          if constexpr (DIM == 3) a = add2(a, pair(Fz, i));
+          put2(acc, i, a);
         }
         ph_prev = pr.q[4];
         if constexpr (DIM < 3) {
@@ -784,9 +789,10 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
         read_row<RECON>(sWj, wx, a0);
         read_row<RECON>(ringk(1), wx, b1);
 #pragma unroll
-        for (int v = 0; v < 6; v++) {
-          ys_m[v] = ppm_slope(c2[v], c1[v], a0[v]);
-          ys_0[v] = ppm_slope(c1[v], a0[v], b1[v]);
+        for (int i = 0; i < 3; i++) {
+          const float2 d = sub2(pair(a0, i), pair(c1, i));
+          put2(ys_m, i, ppm_slope2(sub2(pair(c1, i), pair(c2, i)), d));
+          put2(ys_0, i, ppm_slope2(d, sub2(pair(b1, i), pair(a0, i))));
         }
         ys_ready = true;
       }
@@ -795,11 +801,15 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
       float p2v[6];
       read_row<RECON>(ringk(2), wx, p2v);
 #pragma unroll
-      for (int v = 0; v < 6; v++) {
-        const float yp = ppm_slope(c[v], p[v], p2v[v]);
-        ppm_incs_d(m[v], c[v], p[v], ys_m[v], ys_0[v], yp, su_y[v], sd_y[v]);
-        ys_m[v] = ys_0[v];
-        ys_0[v] = yp;
+      for (int i = 0; i < 3; i++) {
+        const float2 cc = pair(c, i), pp = pair(p, i), dr = sub2(pp, cc);
+        const float2 sp = ppm_slope2(dr, sub2(pair(p2v, i), pp)), s0 = pair(ys_0, i);
+        float2 u, d;
+        ppm_edges2(sub2(cc, pair(m, i)), dr, pair(ys_m, i), s0, sp, u, d);
+        put2(su_y, i, u);
+        put2(sd_y, i, d);
+        put2(ys_m, i, s0);
+        put2(ys_0, i, sp);
       }
     };
 
@@ -811,6 +821,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
       float c[7], m[7], p[7], m2[7], p2[7], su[6], sd[6];
       read_row<RECON>(sWj, wx, c);
       with_cs(c, P);
+      const CellInv ci = cell_inv(c);
       read_row<RECON>(ringk(-1), wx, m);
       read_row<RECON>(ringk(1), wx, p);
       if constexpr (YCARRY) {
@@ -818,7 +829,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
         (void)p2;
         y_edges(m, c, p, su, sd);
       } else {
-        axis_edges<RECON, ISEN, false>(m2, m, c, p, p2, P.inv_gamma, su, sd);
+        axis_edges<RECON, ISEN>(m2, m, c, p, p2, ci, P.inv_gamma, su, sd);
       }
       if (yg_lo) {
 #pragma unroll
@@ -835,7 +846,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
         face_state(g, sd, -1.f, ylo);
         riemann<1>(yhi_prev, ylo, P, Fy, flagged_prev);
 #pragma unroll
-        for (int v = 0; v < 8; v++) acc[v] -= Fy[v];
+        for (int i = 0; i < 4; i++) put2(acc, i, sub2(pair(acc, i), pair(Fy, i)));
         const size_t o = (size_t)(j - 1) * nx + gx;
         float4 na, nb;
         update_cell(__ldg(u1 + o), __ldg(u2 + o), acc, ph_prev, dtdx, P, na, nb);
@@ -850,6 +861,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
     float c[7];
     read_row<RECON>(sWj, wx, c);
     with_cs(c, P);
+    const CellInv ci = cell_inv(c);
     float su[2][6], sd[2][6];
     float conv = 0.f, jump = -INFINITY;
     {
@@ -860,7 +872,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
         read_row<RECON>(sWj, wx - 2, m2);
         read_row<RECON>(sWj, wx + 2, p2);
       }
-      axis_edges<RECON, ISEN, false>(m2, m, c, p, p2, P.inv_gamma, su[0], sd[0]);
+      axis_edges<RECON, ISEN>(m2, m, c, p, p2, ci, P.inv_gamma, su[0], sd[0]);
       conv += p[1] - m[1];
       jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
       read_row<RECON>(ringk(-1), wx, m);
@@ -868,13 +880,13 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
       if constexpr (YCARRY) {
         y_edges(m, c, p, su[1], sd[1]);
       } else {
-        axis_edges<RECON, ISEN, false>(m2, m, c, p, p2, P.inv_gamma, su[1], sd[1]);
+        axis_edges<RECON, ISEN>(m2, m, c, p, p2, ci, P.inv_gamma, su[1], sd[1]);
       }
       conv += p[2] - m[2];
       jump = fmaxf(jump, jump_excess(m[4], p[4], P.shock_thresh));
     }
     Pred pr;
-    hancock<2>(c, conv, jump, su, sd, h, P, pr);
+    hancock<2>(c, ci.r, conv, jump, su, sd, h, P, pr);
 
     const bool row_plane = j >= y0 && j < y1;
     if (xg && row_plane) {
@@ -929,7 +941,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
     if (col_t) {
       if (j - 1 >= y0) {
 #pragma unroll
-        for (int v = 0; v < 8; v++) acc[v] -= Fy[v];
+        for (int i = 0; i < 4; i++) put2(acc, i, sub2(pair(acc, i), pair(Fy, i)));
         const size_t o = (size_t)(j - 1) * nx + gx;
         float4 na, nb;
         update_cell(__ldg(u1 + o), __ldg(u2 + o), acc, ph_prev, dtdx, P, na, nb);
@@ -942,12 +954,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
         unpack8(sFlux[tid], sFlux[PX + tid], xl);
         unpack8(sFlux[tid + 1], sFlux[PX + tid + 1], xu);
 #pragma unroll
-        for (int v = 0; v < 8; v++) {
-          float a = xl[v];
-          a -= xu[v];
-          a += Fy[v];
-          acc[v] = a;
-        }
+        for (int i = 0; i < 4; i++) put2(acc, i, add2(sub2(pair(xl, i), pair(xu, i)), pair(Fy, i)));
         ph_prev = pr.q[4];
       }
     }
