@@ -3,7 +3,7 @@
 // The handle stands where the reference's Sim (src/sim.ts:1938) stands behind its Simulation
 // interface (src/sim.ts:465-628): it owns the device state (two float4 arrays per parity, as
 // the reference's 2x2 rgba32f textures, src/sim.ts:2301), the device clock and one stream, and
-// enqueues a step as clock_kernel + sweep_kernel (sweep.cu). run() follows src/ui/api.ts:538:
+// enqueues a step as one kernel (sweep.cu). run() follows src/ui/api.ts:538:
 // batches of steps whose clock is read back between batches; dt never leaves the device.
 #include <cuda_runtime.h>
 
@@ -35,9 +35,10 @@ struct shz_sim {
   shz::SweepMaps maps[2];              // 3D: tensor maps of each parity for the sweep's TMA staging
   int* d_err = nullptr;                // the kernels' error word (a bounded wait that ran out)
   int cur = 0;
-  shz::DevClock* clk = nullptr;
-  unsigned* rates = nullptr;  // two slots
-  int slot = 0;               // slot the next clock kernel reads
+  shz::DevClock* clk = nullptr;  // two copies: a step reads one and writes the other
+  int ccur = 0;                  // the current one
+  unsigned* rates = nullptr;     // three slots: a step reads one, fills the next, empties the third
+  int slot = 0;                  // the slot the next step reads
   double* diag_part = nullptr;
   double* diag_out = nullptr;
   cudaStream_t stream = nullptr;
@@ -160,7 +161,7 @@ int write_clock(shz_sim* s, double t, long long steps) {
   h.max_steps = std::numeric_limits<long long>::max();
   h.held = 0;
   h.bad = 0;
-  CUDA_OR_FAIL(s, cudaMemcpyAsync(s->clk, &h, sizeof h, cudaMemcpyHostToDevice, s->stream));
+  CUDA_OR_FAIL(s, cudaMemcpyAsync(s->clk + s->ccur, &h, sizeof h, cudaMemcpyHostToDevice, s->stream));
   CUDA_OR_FAIL(s, cudaStreamSynchronize(s->stream));
   return 0;
 }
@@ -178,12 +179,13 @@ int check_err(shz_sim* s) {
 }
 
 int read_clock(shz_sim* s, shz::DevClock* h) {
-  CUDA_OR_FAIL(s, cudaMemcpyAsync(h, s->clk, sizeof *h, cudaMemcpyDeviceToHost, s->stream));
+  CUDA_OR_FAIL(s, cudaMemcpyAsync(h, s->clk + s->ccur, sizeof *h, cudaMemcpyDeviceToHost, s->stream));
   CUDA_OR_FAIL(s, cudaStreamSynchronize(s->stream));
   return check_err(s);
 }
 
-// The rate maximum of the current state into the slot the next clock kernel reads.
+// The rate maximum of the current state into the slot the next step reads (the one that step folds
+// into is empty: the last step, or the handle's creation, left it so).
 int refresh_rate(shz_sim* s) {
   CUDA_OR_FAIL(s, shz::launch_rate(s->kp, s->u1[s->cur], s->u2[s->cur], s->ncell, s->rates + s->slot, s->stream));
   s->launches += 2;
@@ -216,24 +218,32 @@ bool wants_tuning(const shz_sim* s) {
          shz::tune::needs(sweep_key(s));
 }
 
+// One step's kernel at depth tz (0: the default), from the current parity, clock copy and rate slot.
+cudaError_t launch_step(shz_sim* s, int tz) {
+  const shz::ClockArgs k{s->clk + s->ccur, s->clk + (s->ccur ^ 1), s->rates + s->slot, s->rates + (s->slot + 1) % 3,
+                         s->rates + (s->slot + 2) % 3};
+  return shz::launch_sweep(s->kp, s->ndim, s->cfg.recon, s->cfg.isentropic != 0, s->u1[s->cur], s->u2[s->cur],
+                           s->u1[1 - s->cur], s->u2[1 - s->cur], k, s->stream, tz, &s->maps[s->cur], s->d_err);
+}
+// What a step wrote becomes current.
+void step_taken(shz_sim* s) {
+  s->cur ^= 1;
+  s->ccur ^= 1;
+  s->slot = (s->slot + 1) % 3;
+}
+
 // One step whose sweep is run once per candidate depth (z planes in 3D, y rows in 2D), timed, the
-// fastest kept. The sweep reads one parity and writes the other (and folds the
-// same rate maximum), so the step's result is that of a single launch. A clock held at its stop time is not tuned on (the sweep would
-// only copy the state).
+// fastest kept. The sweep reads one parity, clock copy and rate slot and writes others, so the
+// step's result is that of a single launch. A clock held at its stop time is not tuned on (the
+// sweep would only copy the state).
 int tuned_step(shz_sim* s) {
-  CUDA_OR_FAIL(s, shz::launch_clock(s->clk, s->rates, s->slot, s->stream));
+  auto launch = [&](const shz::tune::Choice& c) { return launch_step(s, c.tz); };
+  CUDA_OR_FAIL(s, launch_step(s, s->ndim == 3 ? 0 : ROWS_DEFAULT));
   s->launches += 1;
   shz::DevClock h;
-  CUDA_OR_FAIL(s, cudaMemcpyAsync(&h, s->clk, sizeof h, cudaMemcpyDeviceToHost, s->stream));
+  CUDA_OR_FAIL(s, cudaMemcpyAsync(&h, s->clk + (s->ccur ^ 1), sizeof h, cudaMemcpyDeviceToHost, s->stream));
   CUDA_OR_FAIL(s, cudaStreamSynchronize(s->stream));
-  auto launch = [&](const shz::tune::Choice& c) {
-    return shz::launch_sweep(s->kp, s->ndim, s->cfg.recon, s->cfg.isentropic != 0, s->u1[s->cur], s->u2[s->cur],
-                             s->u1[1 - s->cur], s->u2[1 - s->cur], s->clk, s->rates + (s->slot ^ 1), s->stream, c.tz, &s->maps[s->cur], s->d_err);
-  };
-  if (h.held) {
-    CUDA_OR_FAIL(s, launch(shz::tune::Choice{}));
-    s->launches += 1;
-  } else {
+  if (!h.held) {
     std::vector<shz::tune::Choice> cands;
     if (s->ndim == 3) {
       for (int tz : {shz::SWEEP_TZ_DEFAULT, 32, 128, 256}) {
@@ -255,8 +265,7 @@ int tuned_step(shz_sim* s) {
     CUDA_OR_FAIL(s, shz::tune::choose(sweep_key(s), cands, launch, s->stream, reps, &best));
     s->launches += (long long)cands.size() * (1 + reps);
   }
-  s->cur ^= 1;
-  s->slot ^= 1;
+  step_taken(s);
   return 0;
 }
 
@@ -267,13 +276,9 @@ int enqueue_steps(shz_sim* s, int n) {
       if (rc) return rc;
       continue;
     }
-    CUDA_OR_FAIL(s, shz::launch_clock(s->clk, s->rates, s->slot, s->stream));
-    CUDA_OR_FAIL(s, shz::launch_sweep(s->kp, s->ndim, s->cfg.recon, s->cfg.isentropic != 0, s->u1[s->cur], s->u2[s->cur],
-                                      s->u1[1 - s->cur], s->u2[1 - s->cur], s->clk, s->rates + (s->slot ^ 1), s->stream,
-                                      sweep_tz(s), &s->maps[s->cur], s->d_err));
-    s->launches += 2;
-    s->cur ^= 1;
-    s->slot ^= 1;
+    CUDA_OR_FAIL(s, launch_step(s, sweep_tz(s)));
+    s->launches += 1;
+    step_taken(s);
   }
   return 0;
 }
@@ -365,14 +370,15 @@ int shz_create(const shz_config* cfg, shz_sim** out) {
   }
   const int dblocks = shz::diag_blocks(s->ncell);
   if (cudaMalloc(&s->d_err, sizeof(int)) != cudaSuccess || cudaMemset(s->d_err, 0, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&s->clk, sizeof(shz::DevClock)) != cudaSuccess || cudaMalloc(&s->rates, 2 * sizeof(unsigned)) != cudaSuccess ||
+      cudaMalloc(&s->clk, 2 * sizeof(shz::DevClock)) != cudaSuccess ||
+      cudaMalloc(&s->rates, 3 * sizeof(unsigned)) != cudaSuccess ||
       cudaMalloc(&s->diag_part, (size_t)dblocks * 16 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&s->diag_out, 16 * sizeof(double)) != cudaSuccess) {  // the totals or the extended channels
     cudaGetLastError();
     fail(s, SHZ_E_OOM, "clock / reduction buffers do not fit");
     return bail(SHZ_E_OOM);
   }
-  cudaMemsetAsync(s->rates, 0, 2 * sizeof(unsigned), s->stream);
+  cudaMemsetAsync(s->rates, 0, 3 * sizeof(unsigned), s->stream);
   if (write_clock(s, 0.0, 0) != 0) return bail(SHZ_E_CUDA);
   *out = s;
   return SHZ_OK;
@@ -510,7 +516,7 @@ int shz_set_t_end(shz_sim* s, double t_end) {
   if (!s) return SHZ_E_CONFIG;
   DeviceScope ds_(s->device);
   s->cfg.t_end = t_end;
-  CUDA_OR_FAIL(s, cudaMemcpyAsync(&s->clk->t_end, &s->cfg.t_end, sizeof(double), cudaMemcpyHostToDevice, s->stream));
+  CUDA_OR_FAIL(s, cudaMemcpyAsync(&s->clk[s->ccur].t_end, &s->cfg.t_end, sizeof(double), cudaMemcpyHostToDevice, s->stream));
   CUDA_OR_FAIL(s, cudaStreamSynchronize(s->stream));
   return 0;
 }
@@ -543,7 +549,7 @@ int shz_run(shz_sim* s, const shz_run_opts* o, shz_run_result* r) {
   const double t_end_was = s->cfg.t_end;
   const double stop = has_until ? std::min(o->until, t_end_was) : t_end_was;
   if (stop != t_end_was) {
-    CUDA_OR_FAIL(s, cudaMemcpyAsync(&s->clk->t_end, &stop, sizeof(double), cudaMemcpyHostToDevice, s->stream));
+    CUDA_OR_FAIL(s, cudaMemcpyAsync(&s->clk[s->ccur].t_end, &stop, sizeof(double), cudaMemcpyHostToDevice, s->stream));
   }
   int stopped = -1;
   int grow = 1;
@@ -577,7 +583,7 @@ int shz_run(shz_sim* s, const shz_run_opts* o, shz_run_result* r) {
     grow = std::min(grow * 2, 256);
   }
   if (stop != t_end_was) {
-    cudaMemcpyAsync(&s->clk->t_end, &t_end_was, sizeof(double), cudaMemcpyHostToDevice, s->stream);
+    cudaMemcpyAsync(&s->clk[s->ccur].t_end, &t_end_was, sizeof(double), cudaMemcpyHostToDevice, s->stream);
     cudaStreamSynchronize(s->stream);
   }
   if (rc) return rc;
@@ -692,17 +698,12 @@ int shz_profile(shz_sim* s, int32_t n, shz_profile_result* out) {
       if (rc == 0) CUDA_OR_FAIL(s, cudaEventRecord(ev[2 + 2 * i], s->stream));
       continue;
     }
-    cudaError_t e = shz::launch_clock(s->clk, s->rates, s->slot, s->stream);
-    if (e == cudaSuccess) e = cudaEventRecord(ev[1 + 2 * i], s->stream);
-    if (e == cudaSuccess)
-      e = shz::launch_sweep(s->kp, s->ndim, s->cfg.recon, s->cfg.isentropic != 0, s->u1[s->cur], s->u2[s->cur],
-                            s->u1[1 - s->cur], s->u2[1 - s->cur], s->clk, s->rates + (s->slot ^ 1), s->stream,
-                            sweep_tz(s), &s->maps[s->cur], s->d_err);
+    cudaError_t e = cudaEventRecord(ev[1 + 2 * i], s->stream);
+    if (e == cudaSuccess) e = launch_step(s, sweep_tz(s));
     if (e == cudaSuccess) e = cudaEventRecord(ev[2 + 2 * i], s->stream);
     if (e != cudaSuccess) rc = fail(s, SHZ_E_CUDA, "profile step %d: %s", i, cudaGetErrorString(e));
-    s->launches += 2;
-    s->cur ^= 1;
-    s->slot ^= 1;
+    s->launches += 1;
+    step_taken(s);
   }
   if (rc == 0) {
     cudaError_t e = cudaEventSynchronize(ev[2 * (size_t)n]);

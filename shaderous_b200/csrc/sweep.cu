@@ -5,12 +5,17 @@
 // (hydro/rates.wgsl), the dt reduction and clock (gpu/reduce.wgsl, hydro/clock.wgsl), the
 // Hancock predictor (hydro/predict.wgsl -> predictor.wgsl) and the update
 // (hydro/update.wgsl -> tile.wgsl, flux.wgsl, riemann/hllc.wgsl, advance.wgsl, dual_energy.wgsl).
-// Here a step is clock_kernel (one thread: dt from the last sweep's rate maximum, the float64
-// clock advanced) and sweep_kernel, which reads each cell's conserved state once and in one
+// Here a step is one kernel. Every CTA forms dt from the last sweep's rate maximum (step_clock; one
+// thread of the grid advances the float64 clock), reads each cell's conserved state once and in one
 // pass recovers primitives, forms limited edge increments, takes the Hancock half step, solves
 // each face's Riemann problem once, applies the conservative update with the dual-energy
 // switch, writes the new state, and folds the new state's signal rate into the next step's
 // maximum (warp shuffles, then one atomicMax per CTA on the float's bits).
+//
+// Small grids are bound by the chain of launches. With the clock a kernel of its own, a step took
+// 10.7 us on a tube of 512 cells and 13.4 us on a 64^2 grid (runs of 64 steps); with the clock in the
+// sweep, and the next step's launch overlapped with this one's work (programmatic dependent launch:
+// step_clock waits for the step before), 6.5 and 8.6 us. Large grids take the same time either way.
 //
 // Decomposition: a CTA owns a TX x TY column of cells and marches it along z through tz planes
 // (2.5D). Its threads are the column's TX x TY cells and one a halo cell across each of its four sides
@@ -158,11 +163,51 @@ __device__ __forceinline__ void block_max_to(float v, float* sRed, unsigned* out
 
 __device__ __forceinline__ float rate_guard(float r) { return (r == r) ? r : __int_as_float(0x7f800000); }
 
+// The clock of a step, formed by every CTA: dt from the rate maximum that the last sweep (or
+// rate_kernel) left (clock.wgsl:38-147, in the reference's CPU form hydro.ts:382
+// dt = min(cfl dx / rate, t_end - t)). A rate that is NaN or infinite marks the clock bad and holds it.
+// The grid's first thread writes the clock advanced by the step, in float64, to the other of the
+// clock's two copies, and empties the rate slot that the next sweep folds into: nothing that a CTA
+// of this launch reads is written in it, so a launch repeated in place gives the same clock and state.
+// The wait comes first: everything read from here on may be the step before's output; then the
+// step after may be launched (it waits likewise for this grid to end).
+struct StepDt {
+  double dt;
+  bool held;
+};
+__device__ __forceinline__ StepDt step_clock(const ClockArgs& K) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const DevClock c = *K.in;
+  const float rate = __uint_as_float(*K.rate);
+  const bool bad = c.bad || !(rate == rate) || isinf(rate);
+  double dt = fmin(c.cfl_dx / fmax((double)rate, 1e-30), c.dt_max);
+  if (c.t_end < HUGE_VAL) {
+    const double rem = c.t_end - c.t;
+    dt = rem <= 1e-12 * fabs(c.t_end) ? 0.0 : fmin(dt, rem);
+  }
+  if (bad) dt = 0.0;
+  const bool held = !(dt > 0.0);
+  if (threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) {
+    DevClock o = c;
+    o.bad = bad ? 1 : 0;
+    o.dt = dt;
+    o.held = held ? 1 : 0;
+    if (!held) {
+      o.t = c.t + dt;
+      o.steps = c.steps + 1;
+      o.last_dt = dt;
+    }
+    *K.out = o;
+    *K.rate_next = 0u;
+  }
+  return {dt, held};
+}
+
 template <int DIM, int RECON, bool ISEN>
 __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, RECON>::MAXREG))
     sweep_kernel(const KParams P, const float4* __restrict__ u1, const float4* __restrict__ u2, float4* __restrict__ o1,
-                 float4* __restrict__ o2, const DevClock* __restrict__ clk, unsigned* __restrict__ rate_out, int tz,
-                 const __grid_constant__ CUtensorMap tm1, const __grid_constant__ CUtensorMap tm2, int zofs, int use_tma,
+                 float4* __restrict__ o2, const ClockArgs K, int tz, const __grid_constant__ CUtensorMap tm1, const __grid_constant__ CUtensorMap tm2, int zofs, int use_tma,
                  int* __restrict__ err) {
   using G = Geo<DIM, RECON>;
   constexpr int H = G::H, ZH = G::ZH, PN = G::PN, WN = G::WN, WC = G::WC, TX = G::TX, TY = G::TY;
@@ -203,13 +248,14 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
   const bool xface_t = row_t && lx >= 0 && gx <= nx;  // solves the x face below gx
   const bool yface_t = (DIM >= 2) && col_t && ly >= 0 && gy <= ny;
 
-  const double dt = clk->dt;
-  const float dtdx = (float)(dt / P.dx);
-  const float h = (float)((0.5 * dt) / P.dx);
+  const StepDt st = step_clock(K);
+  unsigned* const rate_out = K.rate_out;
+  const float dtdx = (float)(st.dt / P.dx);
+  const float h = (float)((0.5 * st.dt) / P.dx);
   float rate_max = 0.f;
 
   // A step held at the stop time (dt = 0) leaves the state as it is (clock.wgsl:120-125).
-  if (clk->held) {
+  if (st.held) {
     const int zb = (DIM == 3) ? blockIdx.z * tz : 0;
     const int ze = (DIM == 3) ? min(zb + tz, nz) : 1;
     for (int idx = tid; idx < G::TX * G::TY; idx += G::NT) {
@@ -694,8 +740,7 @@ template <int RECON, bool ISEN>
 // the Kelvin-Helmholtz march ran 4-8 % slower)
 __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
     sweep_rows_kernel(const KParams P, const float4* __restrict__ u1, const float4* __restrict__ u2,
-                      float4* __restrict__ o1, float4* __restrict__ o2, const DevClock* __restrict__ clk,
-                      unsigned* __restrict__ rate_out, int rows) {
+                      float4* __restrict__ o1, float4* __restrict__ o2, const ClockArgs K, int rows) {
   using G = RowGeo<RECON>;
   constexpr int H = G::H, ZH = G::ZH, PX = G::PX, WX = G::WX, WC = G::WC;
   extern __shared__ __align__(128) float smem[];
@@ -714,12 +759,13 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
   const bool xface_t = tid >= 1 && tid <= G::TX + 1 && gx <= nx;       // solves the x face below gx
   const int y0 = blockIdx.y * rows, y1 = min(y0 + rows, ny);
 
-  const double dt = clk->dt;
-  const float dtdx = (float)(dt / P.dx);
-  const float h = (float)((0.5 * dt) / P.dx);
+  const StepDt st = step_clock(K);
+  unsigned* const rate_out = K.rate_out;
+  const float dtdx = (float)(st.dt / P.dx);
+  const float h = (float)((0.5 * st.dt) / P.dx);
   float rate_max = 0.f;
 
-  if (clk->held) {
+  if (st.held) {
     if (col_t)
       for (int y = y0; y < y1; y++) {
         const size_t o = (size_t)y * nx + gx;
@@ -998,32 +1044,6 @@ __global__ void rate_kernel(const KParams P, const float4* __restrict__ u1, cons
   block_max_to<256>(m, sRed, out);
 }
 
-// One thread: dt from the rate maximum (clock.wgsl:38-147, in the reference's CPU form
-// hydro.ts:382 dt = min(cfl dx / rate, t_end - t)), the clock advanced by the step in float64.
-// A rate that is NaN or infinite marks the clock bad and holds it.
-__global__ void clock_kernel(DevClock* clk, unsigned* rates, int slot) {
-  const float rate = __uint_as_float(rates[slot]);
-  rates[slot ^ 1] = 0u;
-  const double t = clk->t;
-  double dt = clk->cfl_dx / fmax((double)rate, 1e-30);
-  if (!(rate == rate) || isinf(rate)) clk->bad = 1;
-  dt = fmin(dt, clk->dt_max);
-  const double te = clk->t_end;
-  if (te < HUGE_VAL) {
-    const double rem = te - t;
-    if (rem <= 1e-12 * fabs(te)) dt = 0.0;
-    else dt = fmin(dt, rem);
-  }
-  if (clk->bad) dt = 0.0;
-  clk->dt = dt;
-  clk->held = dt > 0.0 ? 0 : 1;
-  if (dt > 0.0) {
-    clk->t = t + dt;
-    clk->steps += 1;
-    clk->last_dt = dt;
-  }
-}
-
 __global__ void zero_kernel(unsigned* p) { *p = 0u; }
 
 // Compensated (Neumaier) float64 accumulation.
@@ -1138,10 +1158,26 @@ cudaError_t launch_diag_ext(const KParams& P, const float4* u1, const float4* u2
   return cudaGetLastError();
 }
 
+// A launch that may begin before the kernel ahead of it in the stream has ended (programmatic stream
+// serialization); step_clock waits for that kernel before anything is read.
+template <typename... KA, typename... A>
+static cudaError_t launch_after(void (*k)(KA...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, KA(a)...);
+}
+
 template <int DIM, int RECON, bool ISEN>
 static cudaError_t launch_sweep_t(const KParams& P, const float4* u1, const float4* u2, float4* o1, float4* o2,
-                                  const DevClock* clk, unsigned* rate_out, int tz, const SweepMaps* maps, int* err,
-                                  cudaStream_t s) {
+                                  const ClockArgs& K, int tz, const SweepMaps* maps, int* err, cudaStream_t s) {
   using G = Geo<DIM, RECON>;
   static bool configured = false;
   if (!configured) {
@@ -1158,82 +1194,78 @@ static cudaError_t launch_sweep_t(const KParams& P, const float4* u1, const floa
             DIM == 3 ? (P.n[2] + tz - 1) / tz : 1);
   static const CUtensorMap none{};
   const bool tma = DIM == 3 && maps && maps->valid;
-  sweep_kernel<DIM, RECON, ISEN><<<grid, G::NT, G::SMEM_BYTES, s>>>(P, u1, u2, o1, o2, clk, rate_out, tz,
-                                                                    tma ? maps->u1 : none, tma ? maps->u2 : none,
-                                                                    tma ? maps->zofs : 0, tma ? 1 : 0, err);
-  return cudaGetLastError();
+  return launch_after(sweep_kernel<DIM, RECON, ISEN>, grid, G::NT, G::SMEM_BYTES, s, P, u1, u2, o1, o2, K, tz,
+                      tma ? maps->u1 : none, tma ? maps->u2 : none, tma ? maps->zofs : 0, tma ? 1 : 0, err);
 }
 
 template <int DIM, int RECON>
 static cudaError_t launch_sweep_r(const KParams& P, bool isen, const float4* u1, const float4* u2, float4* o1, float4* o2,
-                                  const DevClock* clk, unsigned* rate_out, int tz, const SweepMaps* maps, int* err,
-                                  cudaStream_t s) {
+                                  const ClockArgs& K, int tz, const SweepMaps* maps, int* err, cudaStream_t s) {
   if constexpr (RECON == R_PPM) {
-    return launch_sweep_t<DIM, RECON, false>(P, u1, u2, o1, o2, clk, rate_out, tz, maps, err, s);
+    return launch_sweep_t<DIM, RECON, false>(P, u1, u2, o1, o2, K, tz, maps, err, s);
   } else {
-    return isen ? launch_sweep_t<DIM, RECON, true>(P, u1, u2, o1, o2, clk, rate_out, tz, maps, err, s)
-                : launch_sweep_t<DIM, RECON, false>(P, u1, u2, o1, o2, clk, rate_out, tz, maps, err, s);
+    return isen ? launch_sweep_t<DIM, RECON, true>(P, u1, u2, o1, o2, K, tz, maps, err, s)
+                : launch_sweep_t<DIM, RECON, false>(P, u1, u2, o1, o2, K, tz, maps, err, s);
   }
 }
 
 template <int DIM>
 static cudaError_t launch_sweep_d(const KParams& P, int recon, bool isen, const float4* u1, const float4* u2, float4* o1,
-                                  float4* o2, const DevClock* clk, unsigned* rate_out, int tz, const SweepMaps* maps,
+                                  float4* o2, const ClockArgs& K, int tz, const SweepMaps* maps,
                                   int* err, cudaStream_t s) {
   switch (recon) {
-    case R_MINMOD: return launch_sweep_r<DIM, R_MINMOD>(P, isen, u1, u2, o1, o2, clk, rate_out, tz, maps, err, s);
-    case R_MC: return launch_sweep_r<DIM, R_MC>(P, isen, u1, u2, o1, o2, clk, rate_out, tz, maps, err, s);
-    case R_VANLEER: return launch_sweep_r<DIM, R_VANLEER>(P, isen, u1, u2, o1, o2, clk, rate_out, tz, maps, err, s);
-    case R_KOREN: return launch_sweep_r<DIM, R_KOREN>(P, isen, u1, u2, o1, o2, clk, rate_out, tz, maps, err, s);
-    case R_PPM: return launch_sweep_r<DIM, R_PPM>(P, isen, u1, u2, o1, o2, clk, rate_out, tz, maps, err, s);
+    case R_MINMOD: return launch_sweep_r<DIM, R_MINMOD>(P, isen, u1, u2, o1, o2, K, tz, maps, err, s);
+    case R_MC: return launch_sweep_r<DIM, R_MC>(P, isen, u1, u2, o1, o2, K, tz, maps, err, s);
+    case R_VANLEER: return launch_sweep_r<DIM, R_VANLEER>(P, isen, u1, u2, o1, o2, K, tz, maps, err, s);
+    case R_KOREN: return launch_sweep_r<DIM, R_KOREN>(P, isen, u1, u2, o1, o2, K, tz, maps, err, s);
+    case R_PPM: return launch_sweep_r<DIM, R_PPM>(P, isen, u1, u2, o1, o2, K, tz, maps, err, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
 template <int RECON, bool ISEN>
 static cudaError_t launch_rows_t(const KParams& P, const float4* u1, const float4* u2, float4* o1, float4* o2,
-                                 const DevClock* clk, unsigned* rate_out, int rows, cudaStream_t s) {
+                                 const ClockArgs& K, int rows, cudaStream_t s) {
   using G = RowGeo<RECON>;
   static_assert(G::SMEM_BYTES <= 48 * 1024, "the row march fits the default shared-memory limit");
   dim3 grid((P.n[0] + G::TX - 1) / G::TX, (P.n[1] + rows - 1) / rows, 1);
-  sweep_rows_kernel<RECON, ISEN><<<grid, G::NT, G::SMEM_BYTES, s>>>(P, u1, u2, o1, o2, clk, rate_out, rows);
-  return cudaGetLastError();
+  return launch_after(sweep_rows_kernel<RECON, ISEN>, grid, G::NT, G::SMEM_BYTES, s, P, u1, u2, o1, o2, K, rows);
 }
 
 template <int RECON>
 static cudaError_t launch_rows_r(const KParams& P, bool isen, const float4* u1, const float4* u2, float4* o1, float4* o2,
-                                 const DevClock* clk, unsigned* rate_out, int rows, cudaStream_t s) {
+                                 const ClockArgs& K, int rows, cudaStream_t s) {
   if constexpr (RECON == R_PPM) {
-    return launch_rows_t<RECON, false>(P, u1, u2, o1, o2, clk, rate_out, rows, s);
+    return launch_rows_t<RECON, false>(P, u1, u2, o1, o2, K, rows, s);
   } else {
-    return isen ? launch_rows_t<RECON, true>(P, u1, u2, o1, o2, clk, rate_out, rows, s)
-                : launch_rows_t<RECON, false>(P, u1, u2, o1, o2, clk, rate_out, rows, s);
+    return isen ? launch_rows_t<RECON, true>(P, u1, u2, o1, o2, K, rows, s)
+                : launch_rows_t<RECON, false>(P, u1, u2, o1, o2, K, rows, s);
   }
 }
 
 static cudaError_t launch_rows(const KParams& P, int recon, bool isen, const float4* u1, const float4* u2, float4* o1,
-                               float4* o2, const DevClock* clk, unsigned* rate_out, int rows, cudaStream_t s) {
+                               float4* o2, const ClockArgs& K, int rows, cudaStream_t s) {
   switch (recon) {
-    case R_MINMOD: return launch_rows_r<R_MINMOD>(P, isen, u1, u2, o1, o2, clk, rate_out, rows, s);
-    case R_MC: return launch_rows_r<R_MC>(P, isen, u1, u2, o1, o2, clk, rate_out, rows, s);
-    case R_VANLEER: return launch_rows_r<R_VANLEER>(P, isen, u1, u2, o1, o2, clk, rate_out, rows, s);
-    case R_KOREN: return launch_rows_r<R_KOREN>(P, isen, u1, u2, o1, o2, clk, rate_out, rows, s);
-    case R_PPM: return launch_rows_r<R_PPM>(P, isen, u1, u2, o1, o2, clk, rate_out, rows, s);
+    case R_MINMOD: return launch_rows_r<R_MINMOD>(P, isen, u1, u2, o1, o2, K, rows, s);
+    case R_MC: return launch_rows_r<R_MC>(P, isen, u1, u2, o1, o2, K, rows, s);
+    case R_VANLEER: return launch_rows_r<R_VANLEER>(P, isen, u1, u2, o1, o2, K, rows, s);
+    case R_KOREN: return launch_rows_r<R_KOREN>(P, isen, u1, u2, o1, o2, K, rows, s);
+    case R_PPM: return launch_rows_r<R_PPM>(P, isen, u1, u2, o1, o2, K, rows, s);
     default: return cudaErrorInvalidValue;
   }
 }
 
 cudaError_t launch_sweep(const KParams& P, int ndim, int recon, bool isen, const float4* u1, const float4* u2, float4* o1,
-                         float4* o2, const DevClock* clk, unsigned* rate_out, cudaStream_t s, int tz,
+                         float4* o2, const ClockArgs& K, cudaStream_t s, int tz,
                          const SweepMaps* maps, int* err) {
   switch (ndim) {
-    case 1: return launch_sweep_d<1>(P, recon, isen, u1, u2, o1, o2, clk, rate_out, 1, nullptr, err, s);
+    case 1: return launch_sweep_d<1>(P, recon, isen, u1, u2, o1, o2, K, 1, nullptr, err, s);
     case 2:
       // tz > 0: the march along y with tz rows a CTA; else the tile form
-      return tz > 0 ? launch_rows(P, recon, isen, u1, u2, o1, o2, clk, rate_out, tz, s)
-                    : launch_sweep_d<2>(P, recon, isen, u1, u2, o1, o2, clk, rate_out, 1, nullptr, err, s);
+      return tz > 0 ? launch_rows(P, recon, isen, u1, u2, o1, o2, K, tz, s)
+                    : launch_sweep_d<2>(P, recon, isen, u1, u2, o1, o2, K, 1, nullptr, err, s);
     case 3:
-      return launch_sweep_d<3>(P, recon, isen, u1, u2, o1, o2, clk, rate_out, tz > 0 ? tz : SWEEP_TZ_DEFAULT, maps,
+      return launch_sweep_d<3>(P, recon, isen, u1, u2, o1, o2, K, tz > 0 ? tz : SWEEP_TZ_DEFAULT, maps,
                                err, s);
     default: return cudaErrorInvalidValue;
   }
@@ -1256,11 +1288,6 @@ cudaError_t launch_rate(const KParams& P, const float4* u1, const float4* u2, si
   if (blocks > 148 * 8) blocks = 148 * 8;
   if (blocks < 1) blocks = 1;
   rate_kernel<<<blocks, 256, 0, s>>>(P, u1, u2, ncell, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_clock(DevClock* clk, unsigned* rates, int slot, cudaStream_t s) {
-  clock_kernel<<<1, 1, 0, s>>>(clk, rates, slot);
   return cudaGetLastError();
 }
 

@@ -30,11 +30,20 @@ bool encode_sweep_maps(SweepMaps* m, const float4* base1, const float4* base2, i
 // staging path and the per-cell loads give the same primitives). err: the kernel's error word (a
 // bounded wait for a copy that ran out), or null.
 constexpr int SWEEP_TZ_DEFAULT = 64;
+// A step's clock and rate words: `in` and `rate` as the last step left them, `out` the other copy of the
+// clock, `rate_out` the (empty) slot this step folds its rates into, `rate_next` the third slot,
+// emptied for the step after.
+struct ClockArgs {
+  const DevClock* in;
+  DevClock* out;
+  const unsigned* rate;
+  unsigned* rate_out;
+  unsigned* rate_next;
+};
 cudaError_t launch_sweep(const KParams& P, int ndim, int recon, bool isen, const float4* u1, const float4* u2, float4* o1,
-                         float4* o2, const DevClock* clk, unsigned* rate_out, cudaStream_t s, int tz = 0,
-                         const SweepMaps* maps = nullptr, int* err = nullptr);
+                         float4* o2, const ClockArgs& K, cudaStream_t s, int tz = 0, const SweepMaps* maps = nullptr,
+                         int* err = nullptr);
 cudaError_t launch_rate(const KParams& P, const float4* u1, const float4* u2, size_t ncell, unsigned* out, cudaStream_t s);
-cudaError_t launch_clock(DevClock* clk, unsigned* rates, int slot, cudaStream_t s);
 int diag_blocks(size_t ncell);
 cudaError_t launch_diag(const KParams& P, const float4* u1, const float4* u2, size_t ncell, double* part, double* out,
                         cudaStream_t s);
