@@ -39,6 +39,7 @@ struct shz_sim {
   int ccur = 0;                  // the current one
   unsigned* rates = nullptr;     // three slots: a step reads one, fills the next, empties the third
   int slot = 0;                  // the slot the next step reads
+  int fit_most = 0, fit_depth = 0;  // the march's depth last fitted, and the bound it was fitted within
   double* diag_part = nullptr;
   double* diag_out = nullptr;
   cudaStream_t stream = nullptr;
@@ -192,12 +193,15 @@ int refresh_rate(shz_sim* s) {
   return 0;
 }
 
-// The autotuner's key of this grid's sweep, and its depth: in 3D the planes a CTA marches along z
-// (0: the default); in 2D the rows a CTA marches along y, 0 for the tile form. Which 2D form runs
+// The autotuner's key of this grid's sweep, and its depth: in 3D the planes a CTA marches along z;
+// in 2D the rows a CTA marches along y, 0 for the tile form. Which 2D form runs
 // is fixed by the grid's size, not by timing: the two forms are different kernels, which agree to
 // rounding (the compiler may contract a multiply and an add differently in each), while every
 // depth of one form is the same kernel and gives the same bits. 2D grids of at least 512 cells a
-// side march along y, at a tuned depth (16 rows untuned); smaller ones take the tile form.
+// side march along y; smaller ones take the tile form. The tuner's choice (64 planes or 16 rows
+// untuned) is the deepest march: the keys are size classes, which grids of many shapes share, and
+// within it the depth that runs is fitted to this grid's own columns (sweep_fit_depth). A pinned
+// depth runs as it is.
 shz::tune::Key sweep_key(const shz_sim* s) {
   return shz::tune::Key{shz::tune::K_UNIFORM_SWEEP, s->ndim, s->cfg.recon,
                         (s->cfg.isentropic != 0 && s->cfg.recon != SHZ_RECON_PPM) ? 1 : 0,
@@ -205,12 +209,19 @@ shz::tune::Key sweep_key(const shz_sim* s) {
 }
 constexpr int ROWS_MIN_SIDE = 512, ROWS_DEFAULT = 16;
 bool rows_form(const shz_sim* s) { return s->ndim == 2 && s->cfg.n[0] >= ROWS_MIN_SIDE && s->cfg.n[1] >= ROWS_MIN_SIDE; }
-int sweep_tz(const shz_sim* s) {
+int fit_depth(shz_sim* s, int most) {
+  if (s->fit_most != most) {
+    s->fit_depth = shz::sweep_fit_depth(s->ndim, s->cfg.n, most);
+    s->fit_most = most;
+  }
+  return s->fit_depth;
+}
+int default_depth(const shz_sim* s) { return s->ndim == 3 ? shz::SWEEP_TZ_DEFAULT : ROWS_DEFAULT; }
+int sweep_tz(shz_sim* s) {
   shz::tune::Choice c;
   if (s->ndim >= 2 && shz::tune::pinned(shz::tune::K_UNIFORM_SWEEP, &c)) return c.tz;
-  if (s->ndim == 3) return shz::tune::lookup(sweep_key(s), &c) ? c.tz : 0;
-  if (!rows_form(s)) return 0;
-  return shz::tune::lookup(sweep_key(s), &c) ? c.tz : ROWS_DEFAULT;
+  if (s->ndim != 3 && !rows_form(s)) return 0;
+  return fit_depth(s, shz::tune::lookup(sweep_key(s), &c) ? c.tz : default_depth(s));
 }
 bool wants_tuning(const shz_sim* s) {
   shz::tune::Choice c;
@@ -218,7 +229,7 @@ bool wants_tuning(const shz_sim* s) {
          shz::tune::needs(sweep_key(s));
 }
 
-// One step's kernel at depth tz (0: the default), from the current parity, clock copy and rate slot.
+// One step's kernel at depth tz (2D: 0 for the tile form), from the current parity, clock copy and rate slot.
 cudaError_t launch_step(shz_sim* s, int tz) {
   const shz::ClockArgs k{s->clk + s->ccur, s->clk + (s->ccur ^ 1), s->rates + s->slot, s->rates + (s->slot + 1) % 3,
                          s->rates + (s->slot + 2) % 3};
@@ -232,13 +243,13 @@ void step_taken(shz_sim* s) {
   s->slot = (s->slot + 1) % 3;
 }
 
-// One step whose sweep is run once per candidate depth (z planes in 3D, y rows in 2D), timed, the
-// fastest kept. The sweep reads one parity, clock copy and rate slot and writes others, so the
+// One step whose sweep is run once per candidate for the deepest march (z planes in 3D, y rows in 2D),
+// each at the depth fitted within it, timed, the fastest kept. The sweep reads one parity, clock copy and rate slot and writes others, so the
 // step's result is that of a single launch. A clock held at its stop time is not tuned on (the
 // sweep would only copy the state).
 int tuned_step(shz_sim* s) {
-  auto launch = [&](const shz::tune::Choice& c) { return launch_step(s, c.tz); };
-  CUDA_OR_FAIL(s, launch_step(s, s->ndim == 3 ? 0 : ROWS_DEFAULT));
+  auto launch = [&](const shz::tune::Choice& c) { return launch_step(s, fit_depth(s, c.tz)); };
+  CUDA_OR_FAIL(s, launch_step(s, fit_depth(s, default_depth(s))));
   s->launches += 1;
   shz::DevClock h;
   CUDA_OR_FAIL(s, cudaMemcpyAsync(&h, s->clk + (s->ccur ^ 1), sizeof h, cudaMemcpyDeviceToHost, s->stream));

@@ -39,6 +39,7 @@
 // (hydro.ts:329-358). Collapsed axes (n = 1) carry no faces: in the reference their two faces
 // carry equal fluxes that cancel.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 
@@ -1269,6 +1270,38 @@ cudaError_t launch_sweep(const KParams& P, int ndim, int recon, bool isen, const
                                err, s);
     default: return cudaErrorInvalidValue;
   }
+}
+
+// A CTA of depth d takes about d + `extra` plane (row) times, `extra` for the planes it only predicts and its
+// first loads; per_sm of them run side by side on an SM, and `share[c]` is what a plane takes with c
+// resident against all per_sm. With few columns the depth is what makes CTAs: a 45 x 52 x 61 grid
+// has 15 columns, and at 64 planes each ran 15 CTAs on 148 SMs; at 7 planes the step takes 38 us and
+// not 171. Where there are many, the depth decides how full the last round of CTAs is. Measured
+// against 64 planes and 16 rows (us a step): 64^3 204 -> 46, 96^3 204 -> 90, 128^3 298 -> 207,
+// 160^3 382 -> 362, 256^3 1380 -> 1339, 2048^2 Koren 211 -> 206. The figures of `extra` and
+// `share` are fitted to depths 2-128 on 24^3-320^3 and 2-64 rows on 64^2-2048^2 (within 4 %).
+int sweep_fit_depth(int ndim, const int n[3], int most) {
+  static const double share3[] = {0.0, 0.65, 1.0}, share2[] = {0.0, 0.46, 0.60, 0.73, 0.87, 1.0};
+  constexpr int SMS = 148;
+  using G = Geo<3, R_MINMOD>;  // (the column's size does not depend on the reconstruction)
+  const bool three = ndim == 3;
+  const long long columns = three ? (long long)((n[0] + G::TX - 1) / G::TX) * ((n[1] + G::TY - 1) / G::TY)
+                                  : (n[0] + RowGeo<R_MINMOD>::TX - 1) / RowGeo<R_MINMOD>::TX;
+  const int len = three ? n[2] : n[1], per_sm = three ? 2 : 5;
+  const double extra = three ? 2.6 : 3.5;
+  const double* share = three ? share3 : share2;
+  double best = 0.0;
+  int depth = 1;
+  for (int d = std::min(most, len); d >= 1; d--) {
+    if ((len + d - 1) / d > 65535 && best > 0.0) break;  // (a grid's y and z extents)
+    const long long per = (columns * ((len + d - 1) / d) + SMS - 1) / SMS;  // CTAs of the fullest SM
+    const double cost = (d + extra) * ((double)(per / per_sm) + share[per % per_sm]);
+    if (best == 0.0 || cost < best) {
+      best = cost;
+      depth = d;
+    }
+  }
+  return depth;
 }
 
 size_t sweep_smem_bytes(int ndim, int recon) {

@@ -43,6 +43,9 @@ struct ClockArgs {
 cudaError_t launch_sweep(const KParams& P, int ndim, int recon, bool isen, const float4* u1, const float4* u2, float4* o1,
                          float4* o2, const ClockArgs& K, cudaStream_t s, int tz = 0, const SweepMaps* maps = nullptr,
                          int* err = nullptr);
+// The march's depth, at most `most`, whose CTAs fill the SMs best (3D: z planes of a column; 2D: y rows of a
+// row segment).
+int sweep_fit_depth(int ndim, const int n[3], int most);
 cudaError_t launch_rate(const KParams& P, const float4* u1, const float4* u2, size_t ncell, unsigned* out, cudaStream_t s);
 int diag_blocks(size_t ncell);
 cudaError_t launch_diag(const KParams& P, const float4* u1, const float4* u2, size_t ncell, double* part, double* out,
