@@ -10,6 +10,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <limits>
@@ -33,7 +34,7 @@ struct shz_sim {
   float4* a2[2] = {nullptr, nullptr};
   int halo_lo = 0, halo_hi = 0;        // stored ghost planes below and above (z faces of code 3)
   shz::SweepMaps maps[2];              // 3D: tensor maps of each parity for the sweep's TMA staging
-  int* d_err = nullptr;                // the kernels' error word (a bounded wait that ran out)
+  int* d_err = nullptr;                // the kernels' error word (a bounded wait that ran out), behind the clocks
   int cur = 0;
   shz::DevClock* clk = nullptr;  // two copies: a step reads one and writes the other
   int ccur = 0;                  // the current one
@@ -167,22 +168,22 @@ int write_clock(shz_sim* s, double t, long long steps) {
   return 0;
 }
 
-// The kernels' error word: a bounded wait inside the sweep that ran out fails the call.
-int check_err(shz_sim* s) {
-  int e = 0;
-  CUDA_OR_FAIL(s, cudaMemcpyAsync(&e, s->d_err, sizeof e, cudaMemcpyDeviceToHost, s->stream));
+// The clock and the kernels' error word, in one copy: a bounded wait inside the sweep that ran out
+// fails the call.
+int read_clock(shz_sim* s, shz::DevClock* h) {
+  struct {
+    shz::DevClock clk[2];
+    int err;
+  } b;
+  static_assert(offsetof(decltype(b), err) == 2 * sizeof(shz::DevClock), "the error word follows the clocks");
+  CUDA_OR_FAIL(s, cudaMemcpyAsync(&b, s->clk, offsetof(decltype(b), err) + sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CUDA_OR_FAIL(s, cudaStreamSynchronize(s->stream));
-  if (e) {
+  *h = b.clk[s->ccur];
+  if (b.err) {
     cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream);
-    return fail(s, SHZ_E_TIMEOUT, "the sweep's bounded wait for a bulk copy ran out (code %d); the state is not valid", e);
+    return fail(s, SHZ_E_TIMEOUT, "the sweep's bounded wait for a bulk copy ran out (code %d); the state is not valid", b.err);
   }
   return 0;
-}
-
-int read_clock(shz_sim* s, shz::DevClock* h) {
-  CUDA_OR_FAIL(s, cudaMemcpyAsync(h, s->clk + s->ccur, sizeof *h, cudaMemcpyDeviceToHost, s->stream));
-  CUDA_OR_FAIL(s, cudaStreamSynchronize(s->stream));
-  return check_err(s);
 }
 
 // The rate maximum of the current state into the slot the next step reads (the one that step folds
@@ -380,8 +381,7 @@ int shz_create(const shz_config* cfg, shz_sim** out) {
     cudaMemsetAsync(s->a2[p], 0, abytes, s->stream);
   }
   const int dblocks = shz::diag_blocks(s->ncell);
-  if (cudaMalloc(&s->d_err, sizeof(int)) != cudaSuccess || cudaMemset(s->d_err, 0, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&s->clk, 2 * sizeof(shz::DevClock)) != cudaSuccess ||
+  if (cudaMalloc(&s->clk, 2 * sizeof(shz::DevClock) + sizeof(int)) != cudaSuccess ||
       cudaMalloc(&s->rates, 3 * sizeof(unsigned)) != cudaSuccess ||
       cudaMalloc(&s->diag_part, (size_t)dblocks * 16 * sizeof(double)) != cudaSuccess ||
       cudaMalloc(&s->diag_out, 16 * sizeof(double)) != cudaSuccess) {  // the totals or the extended channels
@@ -389,6 +389,8 @@ int shz_create(const shz_config* cfg, shz_sim** out) {
     fail(s, SHZ_E_OOM, "clock / reduction buffers do not fit");
     return bail(SHZ_E_OOM);
   }
+  s->d_err = reinterpret_cast<int*>(s->clk + 2);
+  cudaMemsetAsync(s->d_err, 0, sizeof(int), s->stream);
   cudaMemsetAsync(s->rates, 0, 3 * sizeof(unsigned), s->stream);
   if (write_clock(s, 0.0, 0) != 0) return bail(SHZ_E_CUDA);
   *out = s;
@@ -403,7 +405,6 @@ void shz_destroy(shz_sim* s) {
     if (s->a1[p]) cudaFree(s->a1[p]);
     if (s->a2[p]) cudaFree(s->a2[p]);
   }
-  if (s->d_err) cudaFree(s->d_err);
   if (s->clk) cudaFree(s->clk);
   if (s->rates) cudaFree(s->rates);
   if (s->diag_part) cudaFree(s->diag_part);
@@ -563,7 +564,11 @@ int shz_run(shz_sim* s, const shz_run_opts* o, shz_run_result* r) {
     CUDA_OR_FAIL(s, cudaMemcpyAsync(&s->clk[s->ccur].t_end, &stop, sizeof(double), cudaMemcpyHostToDevice, s->stream));
   }
   int stopped = -1;
+  // The first batch is about a millisecond of steps on a small grid (8 us and 8 G cells/s a step), or one
+  // step where a stop time is set and no step has told how far off it is; a look at the clock costs
+  // a small grid's run two or three steps (a tube's 64 steps in 7 batches: 415 us, in one: 241 us).
   int grow = 1;
+  if (!std::isfinite(stop) || last_dt > 0) grow = (int)std::max(1.0, std::min(64.0, 1e-3 / (8e-6 + (double)s->ncell / 8e9)));
   double ms_per_step = 0;  // the batches' pace (api.ts run: batches of about BATCH_MS = 50 ms)
   for (;;) {
     const long long taken = c.steps - start;
@@ -719,7 +724,8 @@ int shz_profile(shz_sim* s, int32_t n, shz_profile_result* out) {
   if (rc == 0) {
     cudaError_t e = cudaEventSynchronize(ev[2 * (size_t)n]);
     if (e != cudaSuccess) rc = fail(s, SHZ_E_CUDA, "profile sync: %s", cudaGetErrorString(e));
-    if (rc == 0) rc = check_err(s);
+    shz::DevClock h;
+    if (rc == 0) rc = read_clock(s, &h);
   }
   if (rc == 0) {
     float tot = 0.f;
