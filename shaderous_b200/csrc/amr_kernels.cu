@@ -850,7 +850,51 @@ cudaError_t amr_launch_regrid(const AmrLaunch& L, const int* rg, const int* list
   return cudaGetLastError();
 }
 
-// The clocks of many grids at once, one thread each: as clock_kernel (sweep.cu), reading grid
+// A state on its way to the host: the blocks of a list gathered into one array a component, so that it
+// crosses in one copy and not in one a block (6,900 leaves of 16^3 took 13,800 copies of 64 KB and
+// 70 ms, 5 us each; gathered, 17 ms, the host link's rate). GRID: into the order of the uniform grid
+// that the blocks tile. Bound by HBM: each cell is read once and written once.
+template <int DIM, bool GRID>
+__global__ void __launch_bounds__(256) amr_gather(const int* __restrict__ list, long long cells, int nr,
+                                                  const float4* __restrict__ u1, const float4* __restrict__ u2,
+                                                  float4* __restrict__ o1, float4* __restrict__ o2) {
+  using namespace amrk;
+  const int n = nr * BS;
+  for (long long o = blockIdx.x * 256LL + threadIdx.x; o < cells; o += gridDim.x * 256LL) {
+    long long src;
+    if constexpr (GRID) {
+      const int i = (int)(o % n), j = (int)(o / n % n), k = DIM == 3 ? (int)(o / ((long long)n * n)) : 0;
+      const int b = ((k / BS) * nr + j / BS) * nr + i / BS;
+      const int l[3] = {i % BS, j % BS, k % BS};
+      src = (long long)__ldg(list + b) * BG<DIM>::CB + cell_ix<DIM>(l);
+    } else {
+      src = (long long)__ldg(list + o / BG<DIM>::CB) * BG<DIM>::CB + o % BG<DIM>::CB;
+    }
+    o1[o] = __ldg(u1 + src);
+    o2[o] = __ldg(u2 + src);
+  }
+}
+
+cudaError_t amr_launch_gather(int ndim, const int* list, int n, const float4* u1, const float4* u2, float4* o1, float4* o2,
+                              cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  const long long cells = (long long)n * (ndim == 3 ? amrk::BG<3>::CB : amrk::BG<2>::CB);
+  const int g = (int)std::min<long long>((cells + 255) / 256, 148 * 8);
+  if (ndim == 3) amr_gather<3, false><<<g, 256, 0, s>>>(list, cells, 1, u1, u2, o1, o2);
+  else amr_gather<2, false><<<g, 256, 0, s>>>(list, cells, 1, u1, u2, o1, o2);
+  return cudaGetLastError();
+}
+
+cudaError_t amr_launch_gather_grid(int ndim, const int* list, int nr, const float4* u1, const float4* u2, float4* o1,
+                                   float4* o2, cudaStream_t s) {
+  const long long n = (long long)nr * amrk::BS, cells = n * n * (ndim == 3 ? n : 1);
+  const int g = (int)std::min<long long>((cells + 255) / 256, 148 * 8);
+  if (ndim == 3) amr_gather<3, true><<<g, 256, 0, s>>>(list, cells, nr, u1, u2, o1, o2);
+  else amr_gather<2, true><<<g, 256, 0, s>>>(list, cells, nr, u1, u2, o1, o2);
+  return cudaGetLastError();
+}
+
+// The clocks of many grids at once, one thread each: as step_clock (sweep.cu), reading grid
 // g's rate from rates[2 g + rslot] and clearing the other slot for the next step; a grid that
 // has taken max_steps steps holds.
 __global__ void clock_multi_kernel(DevClock* __restrict__ clks, unsigned* __restrict__ rates, int rslot, int ngrids,

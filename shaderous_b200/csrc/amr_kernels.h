@@ -113,6 +113,12 @@ cudaError_t amr_launch_diag(const AmrLaunch& L, const int* list, int n, const fl
 // amr_diag_blocks(n) x 13 doubles.
 cudaError_t amr_launch_diag_ext(const AmrLaunch& L, const int* list, int n, const float4* u1, const float4* u2,
                                 double* part, double* out, cudaStream_t s);
+// The state of the blocks in list, one after another (block i's cells at i * 16^ndim) in o1, o2.
+cudaError_t amr_launch_gather(int ndim, const int* list, int n, const float4* u1, const float4* u2, float4* o1, float4* o2,
+                              cudaStream_t s);
+// The state of a grid of nr blocks a side (list: its blocks, x fastest) as the uniform grid's cells.
+cudaError_t amr_launch_gather_grid(int ndim, const int* list, int nr, const float4* u1, const float4* u2, float4* o1,
+                                   float4* o2, cudaStream_t s);
 cudaError_t amr_launch_ghost_map(const AmrLaunch& L, int slot, int* out, cudaStream_t s);
 
 }  // namespace shz

@@ -1192,12 +1192,13 @@ int shz_amr_table(shz_amr* a, int32_t* out) {
 int shz_amr_get_leaves_state(shz_amr* a, float* u1, float* u2) {
   if (!a || !u1 || !u2) return SHZ_E_CONFIG;
   Dev dv(a->device);
-  const size_t bytes = (size_t)a->CB * sizeof(float4);
-  for (int i = 0; i < n_leaves(a); i++) {
-    const size_t s = (size_t)a->h_leaves[i] * a->CB;
-    AMR_CUDA(a, cudaMemcpyAsync(u1 + (size_t)i * a->CB * 4, a->u1[a->cur] + s, bytes, cudaMemcpyDeviceToHost, a->stream));
-    AMR_CUDA(a, cudaMemcpyAsync(u2 + (size_t)i * a->CB * 4, a->u2[a->cur] + s, bytes, cudaMemcpyDeviceToHost, a->stream));
-  }
+  // gathered into the other parity, which between steps holds nothing that is read again (a step, a
+  // re-mesh and a cycle read the current one and write every leaf they leave)
+  float4 *g1 = a->u1[1 - a->cur], *g2 = a->u2[1 - a->cur];
+  const size_t bytes = (size_t)n_leaves(a) * a->CB * sizeof(float4);
+  AMR_CUDA(a, shz::amr_launch_gather(a->cfg.ndim, a->d_leaves, n_leaves(a), a->u1[a->cur], a->u2[a->cur], g1, g2, a->stream));
+  AMR_CUDA(a, cudaMemcpyAsync(u1, g1, bytes, cudaMemcpyDeviceToHost, a->stream));
+  AMR_CUDA(a, cudaMemcpyAsync(u2, g2, bytes, cudaMemcpyDeviceToHost, a->stream));
   AMR_CUDA(a, cudaStreamSynchronize(a->stream));
   return 0;
 }

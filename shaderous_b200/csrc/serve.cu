@@ -540,17 +540,17 @@ int finish(shz_server* s, Engine& e, Grid& G) {
   e.launches += 2;
   double v[9];
   SV_CUDA(s, cudaMemcpyAsync(v, e.d_out, sizeof v, cudaMemcpyDeviceToHost, e.stream));
-  const int CB = e.CB, n = G.req.n, nd = G.req.ndim, nr = n / BS;
-  std::vector<float4> b1, b2;
   if (s->cfg.keep_states) {
-    b1.resize((size_t)G.nblocks * CB);
-    b2.resize((size_t)G.nblocks * CB);
-    for (int b = 0; b < G.nblocks; b++) {
-      SV_CUDA(s, cudaMemcpyAsync(b1.data() + (size_t)b * CB, e.u1[e.cur] + (size_t)G.slots[b] * CB, CB * sizeof(float4),
-                                 cudaMemcpyDeviceToHost, e.stream));
-      SV_CUDA(s, cudaMemcpyAsync(b2.data() + (size_t)b * CB, e.u2[e.cur] + (size_t)G.slots[b] * CB, CB * sizeof(float4),
-                                 cudaMemcpyDeviceToHost, e.stream));
-    }
+    // in the uniform grid's order, gathered into the other parity (between rounds it holds nothing
+    // that is read again)
+    const size_t cells = (size_t)G.nblocks * e.CB;
+    float4 *g1 = e.u1[1 - e.cur], *g2 = e.u2[1 - e.cur];
+    SV_CUDA(s, shz::amr_launch_gather_grid(e.ndim, e.d_glist, G.req.n / BS, e.u1[e.cur], e.u2[e.cur], g1, g2, e.stream));
+    e.launches += 1;
+    G.out1.resize(cells * 4);
+    G.out2.resize(cells * 4);
+    SV_CUDA(s, cudaMemcpyAsync(G.out1.data(), g1, cells * sizeof(float4), cudaMemcpyDeviceToHost, e.stream));
+    SV_CUDA(s, cudaMemcpyAsync(G.out2.data(), g2, cells * sizeof(float4), cudaMemcpyDeviceToHost, e.stream));
   }
   SV_CUDA(s, cudaStreamSynchronize(e.stream));
   const shz::DevClock& c = e.h_clk[G.g];
@@ -566,21 +566,6 @@ int finish(shz_server* s, Engine& e, Grid& G) {
   G.diag.e_tot = v[6];
   G.diag.floored = v[7];
   G.diag.max_mach = v[8];
-  if (s->cfg.keep_states) {
-    const size_t cells = (size_t)n * n * (nd == 3 ? n : 1);
-    G.out1.resize(cells * 4);
-    G.out2.resize(cells * 4);
-    for (int b = 0; b < G.nblocks; b++) {
-      const int bi = b % nr, bj = (b / nr) % nr, bk = nd == 3 ? b / (nr * nr) : 0;
-      for (int t = 0; t < CB; t++) {
-        const int i = bi * BS + t % BS, j = bj * BS + (t / BS) % BS, k = nd == 3 ? bk * BS + t / (BS * BS) : 0;
-        const size_t o = (((size_t)k * n + j) * n + i) * 4;
-        const float4 a = b1[(size_t)b * CB + t], d = b2[(size_t)b * CB + t];
-        G.out1[o] = a.x; G.out1[o + 1] = a.y; G.out1[o + 2] = a.z; G.out1[o + 3] = a.w;
-        G.out2[o] = d.x; G.out2[o + 1] = d.y; G.out2[o + 2] = d.z; G.out2[o + 3] = d.w;
-      }
-    }
-  }
   // idle the clock index and free the slots
   shz::DevClock idle;
   std::memset(&idle, 0, sizeof idle);
