@@ -40,6 +40,10 @@ struct ClockArgs {
   unsigned* rate_out;
   unsigned* rate_next;
 };
+// (the march along y, sweep_rows.cu: segments of ROW_CELLS cells, `rows` rows a CTA)
+constexpr int ROW_CELLS = 126;
+cudaError_t launch_rows(const KParams& P, int recon, bool isen, const float4* u1, const float4* u2, float4* o1, float4* o2,
+                        const ClockArgs& K, int rows, cudaStream_t s);
 cudaError_t launch_sweep(const KParams& P, int ndim, int recon, bool isen, const float4* u1, const float4* u2, float4* o1,
                          float4* o2, const ClockArgs& K, cudaStream_t s, int tz = 0, const SweepMaps* maps = nullptr,
                          int* err = nullptr);

@@ -9,17 +9,37 @@
 #pragma once
 #include "hydro_math.cuh"
 
+#ifdef SHZ_PACKED_PAIRS
+#define SHZ_UNI uni_packed
+#else
+#define SHZ_UNI uni
+#endif
+
 namespace shz {
-namespace uni {
+namespace SHZ_UNI {
 
 // The primitives are kept and read as the pairs (rho vx), (vy vz), (p s); what treats the six alike
-// is written on the pairs.
+// is written on the pairs. With SHZ_PACKED_PAIRS a pair's add, multiply or fma is one instruction of
+// sm_100 (one issue slot for two operations of the same rate); else two.
+#ifdef SHZ_PACKED_PAIRS
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n sub.rn.ftz.f32x2 z, x, y;\n mov.b64 {%0, %1}, z;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+#else
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
 }
+#endif
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 pair(const float* x, int i) { return make_float2(x[2 * i], x[2 * i + 1]); }
 __device__ __forceinline__ void put2(float* x, int i, float2 v) {
@@ -367,5 +387,5 @@ __device__ __forceinline__ void update_cell(const float4 a, const float4 b, cons
   nb = make_float4(E, eint, fmaf(dtdx, acc[6], b.z), b.w);
 }
 
-}  // namespace uni
+}  // namespace SHZ_UNI
 }  // namespace shz
