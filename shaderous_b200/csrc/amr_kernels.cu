@@ -324,18 +324,22 @@ __global__ void __launch_bounds__(NT, MINB) amr_assemble(const KParams* __restri
 // neighbours at its own level, and its images across the domain's faces). The rest of the ghosts
 // are the second pass's (amr_assemble with REST). Every texel gets the same numbers as in the
 // one-pass kernel: the same load, velocity signs and prim_from_cons.
+// parts: the CTAs that share a block, each a part of its texels (assemble_parts; 1 with per-block
+// timesteps, whose rate is the whole block's).
 template <int DIM, bool BINS>
 __global__ void __launch_bounds__(NT, 4) amr_assemble_plain(const KParams* __restrict__ gp, const int* __restrict__ bt,
                                                         const int* __restrict__ list, int n, const float4* __restrict__ u1,
                                                         const float4* __restrict__ u2, float4* __restrict__ w1,
                                                         float4* __restrict__ w2, unsigned* __restrict__ rates, int rslot,
-                                                        const int* __restrict__ bins, float* __restrict__ brate) {
+                                                        const int* __restrict__ bins, float* __restrict__ brate, int parts) {
   __shared__ float sRed[NT / 32];
   constexpr int NS = BG<DIM>::WN - BG<DIM>::CB;
   constexpr int U = 1;  // shell texels a thread resolves, then loads together (more spill in 3D)
-  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+  const int stride = NT * parts;
+  for (int it = blockIdx.x; it < n * parts; it += gridDim.x) {
     float rmax = 0.f;
-    const int slot = __ldg(list + i);
+    const int slot = __ldg(list + it / parts);
+    const int first = (it % parts) * NT + threadIdx.x;
     const int g = bt_at(bt, slot, GRID_WORD);
     const KParams& P = gp[g];
     const bool leaf = leaf_of(bt, slot);
@@ -343,7 +347,7 @@ __global__ void __launch_bounds__(NT, 4) amr_assemble_plain(const KParams* __res
     if (leaf) {
       // a leaf's own cells: u_at's load of its own cell
 #pragma unroll 4
-      for (int t = threadIdx.x; t < BG<DIM>::CB; t += NT) {
+      for (int t = first; t < BG<DIM>::CB; t += stride) {
         const int l[3] = {t & (BS - 1), (t >> 4) & (BS - 1), DIM == 3 ? t >> 8 : 0};
         const size_t c = (size_t)slot * BG<DIM>::CB + t;
         const float4 ua = __ldg(u1 + c), ub = __ldg(u2 + c);
@@ -356,7 +360,7 @@ __global__ void __launch_bounds__(NT, 4) amr_assemble_plain(const KParams* __res
       }
     } else {
       // a parent's (the two-pass form assembles every block): restricted from its children
-      for (int t = threadIdx.x; t < BG<DIM>::CB; t += NT) {
+      for (int t = first; t < BG<DIM>::CB; t += stride) {
         const int l[3] = {t & (BS - 1), (t >> 4) & (BS - 1), DIM == 3 ? t >> 8 : 0};
         const Cons u = u_at<DIM>(bt, u1, u2, slot, l);
         float w[7];
@@ -366,12 +370,12 @@ __global__ void __launch_bounds__(NT, 4) amr_assemble_plain(const KParams* __res
         w2[o] = make_float4(w[4], w[5], w[6], 0.f);
       }
     }
-    for (int i0 = threadIdx.x; i0 < NS; i0 += U * NT) {
+    for (int i0 = first; i0 < NS; i0 += U * stride) {
       long long src[U];
       int dst[U];  // the texel (13 bits), and bits 13-15: the velocity components whose sign flips
 #pragma unroll
       for (int q = 0; q < U; q++) {
-        const int k = i0 + q * NT;
+        const int k = i0 + q * stride;
         src[q] = -1;
         dst[q] = 0;
         if (k < NS) {
@@ -675,17 +679,36 @@ cudaError_t assemble_v(const AmrLaunch& L, int g, const int* list, int n, const 
   }
   return cudaSuccess;
 }
+// The CTAs that share a block in the plain pass: with few blocks (a served batch of 99, a mesh of 736: one
+// and a quarter rounds of 592 CTAs) one CTA a block leaves SMs idle, or the last round nearly empty. 32
+// steps of the mesh of 736: 19.5 -> 18.6 ms.
+int assemble_parts(int ndim, int n, int per_sm) {
+  if (ndim != 3) return 1;
+  const long long slots = 148LL * std::min(per_sm, 4);
+  double best = 0.0;
+  int parts = 1;
+  for (int p = 1; p <= 8; p *= 2) {
+    const double cost = (double)((n * (long long)p + slots - 1) / slots) / p + 0.03 * p;
+    if (best == 0.0 || cost < 0.95 * best) {
+      best = cost;
+      parts = p;
+    }
+  }
+  return parts;
+}
+
 // The split form: the plain pass (own cells and same-level ghosts, 4 CTAs per SM), then the rest
 // of the ghosts with the MINB register budget.
 template <bool BINS>
 cudaError_t assemble_plain(const AmrLaunch& L, const int* list, int n, const float4* u1, const float4* u2,
                            unsigned* rates, int rslot, cudaStream_t s, const int* bins, float* brate,
                            int per_sm = 4) {
-  const int g = grid_for(n, per_sm);
+  const int parts = BINS ? 1 : assemble_parts(L.ndim, n, per_sm);
+  const int g = grid_for(n * parts, per_sm);
   if (L.ndim == 3)
-    amrk::amr_assemble_plain<3, BINS><<<g, amrk::NT, 0, s>>>(L.gp, L.bt, list, n, u1, u2, L.w1, L.w2, rates, rslot, bins, brate);
+    amrk::amr_assemble_plain<3, BINS><<<g, amrk::NT, 0, s>>>(L.gp, L.bt, list, n, u1, u2, L.w1, L.w2, rates, rslot, bins, brate, parts);
   else
-    amrk::amr_assemble_plain<2, BINS><<<g, amrk::NT, 0, s>>>(L.gp, L.bt, list, n, u1, u2, L.w1, L.w2, rates, rslot, bins, brate);
+    amrk::amr_assemble_plain<2, BINS><<<g, amrk::NT, 0, s>>>(L.gp, L.bt, list, n, u1, u2, L.w1, L.w2, rates, rslot, bins, brate, parts);
   return cudaGetLastError();
 }
 template <int MINB>
