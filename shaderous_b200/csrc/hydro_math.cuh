@@ -24,7 +24,7 @@ struct KParams {
 };
 
 // The clock on the device (the reference's Clock, src/hydro/common.wgsl:84-96), advanced by
-// clock_kernel before each sweep: t is the time of the state the sweep in flight produces.
+// each step (step_clock, clock_multi_kernel): t is the time of the state the sweep in flight produces.
 struct DevClock {
   double t;
   double dt;

@@ -4,7 +4,7 @@
 // Each request is a uniform grid of 16^ndim-cell blocks: a level-0 block tree whose rows the
 // server writes into one shared block table, with the request's own parameter and clock index in
 // word 26. An engine per dimensionality owns the shared atlases; a round is `round_steps` steps,
-// each one CUDA graph of three kernels (assemble, clocks, the fused block sweep) over the blocks of
+// each one CUDA graph of three kernels (assemble, clocks, the served grids' block sweep) over the blocks of
 // every running request. Between rounds the
 // host reads the clocks back, finishes the requests that have taken their steps (float64 totals,
 // optionally their state), frees their slots, and admits queued requests whose blocks fit, their
@@ -489,8 +489,9 @@ int enqueue_step(shz_server* s, Engine& e, bool tune_now, long long* launches) {
                                      launches));
   SV_CUDA(s, shz::launch_clock_multi(e.d_clk, e.d_rates, e.rslot, e.gmax, e.stream));
   *launches += 1;
-  SV_CUDA(s, shz::amr_sweep_tuned(e.L, e.d_list, n, e.u1[e.cur], e.u2[e.cur], e.u1[1 - e.cur], e.u2[1 - e.cur], e.d_clk,
-                                  e.stream, tune_now, launches));
+  SV_CUDA(s, shz::launch_grid_sweep(e.L, e.d_list, n, e.u1[e.cur], e.u2[e.cur], e.u1[1 - e.cur], e.u2[1 - e.cur], e.d_clk,
+                                    e.stream));
+  *launches += 1;
   return 0;
 }
 
@@ -501,7 +502,7 @@ int launch_round(shz_server* s, Engine& e) {
   if (e.dirty && (rc = rebuild(s, e))) return rc;
   for (int k = 0; k < s->cfg.round_steps; k++) {
     const int nb = (int)e.h_list.size();
-    if (shz::amr_step_wants_tuning(e.L, nb, nb, 0)) {
+    if (shz::amr_step_wants_tuning(e.L, nb, 0, 0)) {
       long long c = 0;
       if ((rc = enqueue_step(s, e, true, &c))) return rc;
       e.launches += c;
