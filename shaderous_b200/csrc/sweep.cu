@@ -129,8 +129,8 @@ __device__ __forceinline__ void read_w(const float* __restrict__ sWb, int wx, in
 template <int DIM, int RECON, bool ISEN>
 __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, RECON>::MAXREG))
     sweep_kernel(const KParams P, const float4* __restrict__ u1, const float4* __restrict__ u2, float4* __restrict__ o1,
-                 float4* __restrict__ o2, const ClockArgs K, int tz, const __grid_constant__ CUtensorMap tm1, const __grid_constant__ CUtensorMap tm2, int zofs, int use_tma,
-                 int* __restrict__ err) {
+                 float4* __restrict__ o2, const ClockArgs K, int tz, const __grid_constant__ CUtensorMap tm1,
+                 const __grid_constant__ CUtensorMap tm2, int zofs, int use_tma, int* __restrict__ err) {
   using G = Geo<DIM, RECON>;
   constexpr int H = G::H, ZH = G::ZH, PN = G::PN, WN = G::WN, WC = G::WC, TX = G::TX, TY = G::TY;
   extern __shared__ __align__(128) float smem[];
