@@ -406,6 +406,9 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
 #pragma unroll
           for (int v = 0; v < 6; v++) gsu[v] = su[v];
           flagged_prev = false;  // plane 0's faces see plane 0's flags only
+          // (plane ZH, converted at the top of the next turn, takes the slot of plane -1 - ZH, which the
+          // edges above read; the other turns have their face barriers between)
+          __syncthreads();
         } else if (tile_t) {
           Pred g;
 #pragma unroll

@@ -240,6 +240,9 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
 #pragma unroll
         for (int v = 0; v < 6; v++) gsu[v] = su[v];
         flagged_prev = false;  // row 0's faces see row 0's flags only
+        // (row ZH, converted at the top of the next turn, takes the slot of row -1 - ZH, which the
+        // edges above read; the other turns have their face barriers between)
+        __syncthreads();
       } else if (col_t) {
         Pred g;
 #pragma unroll
