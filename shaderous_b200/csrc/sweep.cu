@@ -106,7 +106,7 @@ __device__ __forceinline__ void load_w_plane(const KParams& P, const float4* __r
     const int gx = bc_map(x0 - G::H + lx, P.n[0], P.bc_lo[0], P.bc_hi[0], fx);
     const int gy = (DIM >= 2) ? bc_map(y0 - G::H + ly, P.n[1], P.bc_lo[1], P.bc_hi[1], fy) : 0;
     const ptrdiff_t o = zoff + (ptrdiff_t)gy * P.n[0] + gx;
-    const float4 a = __ldg(u1 + o), b = __ldg(u2 + o);
+    const float4 a = ld_state(u1 + o), b = ld_state(u2 + o);
     float w[6];
     prim6_from_cons(a, b, P, fx, fy, fz, w);
 #pragma unroll
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
       if (cx >= nx || cy >= ny) continue;
       for (int z = zb; z < ze; z++) {
         const size_t o = ((size_t)z * ny + cy) * nx + cx;
-        const float4 a = u1[o], b = u2[o];
+        const float4 a = ld_state(u1 + o), b = ld_state(u2 + o);
         o1[o] = a;
         o2[o] = b;
         rate_max = fmaxf(rate_max, rate_guard(signal_rate(a, b, P)));
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
           for (int i = 0; i < 4; i++) put2(acc, i, sub2(pair(acc, i), pair(Fz, i)));
           const size_t o = ((size_t)(j - 1) * ny + gy) * nx + gx;
           float4 na, nb;
-          update_cell(__ldg(u1 + o), __ldg(u2 + o), acc, ph_prev, dtdx, P, na, nb);
+          update_cell(ld_state(u1 + o), ld_state(u2 + o), acc, ph_prev, dtdx, P, na, nb);
           o1[o] = na;
           o2[o] = nb;
           rate_max = fmaxf(rate_max, rate_guard(signal_rate(na, nb, P)));
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
           for (int i = 0; i < 4; i++) put2(acc, i, sub2(pair(acc, i), pair(Fz, i)));
           const size_t o = ((size_t)(j - 1) * ny + gy) * nx + gx;
           float4 na, nb;
-          update_cell(__ldg(u1 + o), __ldg(u2 + o), acc, ph_prev, dtdx, P, na, nb);
+          update_cell(ld_state(u1 + o), ld_state(u2 + o), acc, ph_prev, dtdx, P, na, nb);
           o1[o] = na;
           o2[o] = nb;
           rate_max = fmaxf(rate_max, rate_guard(signal_rate(na, nb, P)));
@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(Geo<DIM, RECON>::NT) __maxnreg__((Geo<DIM, REC
         if constexpr (DIM < 3) {
           const size_t o = (size_t)gy * nx + gx;
           float4 na, nb;
-          update_cell(__ldg(u1 + o), __ldg(u2 + o), acc, ph_prev, dtdx, P, na, nb);
+          update_cell(ld_state(u1 + o), ld_state(u2 + o), acc, ph_prev, dtdx, P, na, nb);
           o1[o] = na;
           o2[o] = nb;
           rate_max = fmaxf(rate_max, rate_guard(signal_rate(na, nb, P)));

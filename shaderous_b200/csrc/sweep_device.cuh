@@ -48,6 +48,16 @@ __device__ __forceinline__ void block_max_to(float v, float* sRed, unsigned* out
 
 __device__ __forceinline__ float rate_guard(float r) { return (r == r) ? r : __int_as_float(0x7f800000); }
 
+// A cell's state as the last step left it. A sweep may be resident while that step still writes the state
+// (launch_after), so the arrays are not constant for the kernel's life and its reads of them must not
+// be taken for such (ld.global.nc, which __ldg is, and plain reads of const __restrict__ pointers may
+// become): a coherent load, and volatile, so that none is moved ahead of step_clock's wait.
+__device__ __forceinline__ float4 ld_state(const float4* p) {
+  float4 v;
+  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
 // The clock of a step, formed by every CTA: dt from the rate maximum that the last sweep (or
 // rate_kernel) left (clock.wgsl:38-147, in the reference's CPU form hydro.ts:382
 // dt = min(cfl dx / rate, t_end - t)). A rate that is NaN or infinite marks the clock bad and holds it.

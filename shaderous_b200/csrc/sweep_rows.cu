@@ -55,7 +55,7 @@ __device__ __forceinline__ void load_w_row(const KParams& P, const float4* __res
   for (int idx = threadIdx.x; idx < G::WX; idx += G::NT) {
     float fx;
     const int gx = bc_map(x0 - G::H + idx, P.n[0], P.bc_lo[0], P.bc_hi[0], fx);
-    const float4 a = __ldg(u1 + yoff + gx), b = __ldg(u2 + yoff + gx);
+    const float4 a = ld_state(u1 + yoff + gx), b = ld_state(u2 + yoff + gx);
     float w[6];
     prim6_from_cons(a, b, P, fx, fy, 1.f, w);
 #pragma unroll
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
     if (col_t)
       for (int y = y0; y < y1; y++) {
         const size_t o = (size_t)y * nx + gx;
-        const float4 a = u1[o], b = u2[o];
+        const float4 a = ld_state(u1 + o), b = ld_state(u2 + o);
         o1[o] = a;
         o2[o] = b;
         rate_max = fmaxf(rate_max, rate_guard(signal_rate(a, b, P)));
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
         for (int i = 0; i < 4; i++) put2(acc, i, sub2(pair(acc, i), pair(Fy, i)));
         const size_t o = (size_t)(j - 1) * nx + gx;
         float4 na, nb;
-        update_cell(__ldg(u1 + o), __ldg(u2 + o), acc, ph_prev, dtdx, P, na, nb);
+        update_cell(ld_state(u1 + o), ld_state(u2 + o), acc, ph_prev, dtdx, P, na, nb);
         o1[o] = na;
         o2[o] = nb;
         rate_max = fmaxf(rate_max, rate_guard(signal_rate(na, nb, P)));
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
         for (int i = 0; i < 4; i++) put2(acc, i, sub2(pair(acc, i), pair(Fy, i)));
         const size_t o = (size_t)(j - 1) * nx + gx;
         float4 na, nb;
-        update_cell(__ldg(u1 + o), __ldg(u2 + o), acc, ph_prev, dtdx, P, na, nb);
+        update_cell(ld_state(u1 + o), ld_state(u2 + o), acc, ph_prev, dtdx, P, na, nb);
         o1[o] = na;
         o2[o] = nb;
         rate_max = fmaxf(rate_max, rate_guard(signal_rate(na, nb, P)));
