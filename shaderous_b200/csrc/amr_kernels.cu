@@ -18,6 +18,7 @@
 
 #include "amr_device.cuh"
 #include "diag_ext.cuh"
+#include "launch_attr.h"
 
 namespace shz {
 namespace amrk {
@@ -661,9 +662,9 @@ cudaError_t assemble_t(const AmrLaunch& L, int g, const int* list, int n, const 
   auto k = amrk::amr_assemble<DIM, R, MINB, BINS, REST>;
   // the coarse-face table, and in the second pass of the split form also the edge table
   constexpr size_t TB = amrk::Tab<DIM>::BYTES + (REST ? amrk::EdgeTab<DIM>::BYTES : 0);
-  // (set once per instantiation; not a stream operation)
-  static const cudaError_t attr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TB);
-  if (attr != cudaSuccess) return attr;
+  static LaunchAttr attr;
+  const cudaError_t e = attr.set((const void*)k, TB, false);
+  if (e != cudaSuccess) return e;
   const size_t smem = L.per_texel ? 0 : TB;
   k<<<g, amrk::NT, smem, s>>>(L.gp, L.bt, list, n, u1, u2, L.w1, L.w2, rates, rslot, L.per_texel ? 1 : 0, L.p1, L.p2,
                               bins, brate);

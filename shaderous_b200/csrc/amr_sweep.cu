@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "amr_device.cuh"
+#include "launch_attr.h"
 #include "tma.cuh"
 
 namespace shz {
@@ -733,15 +734,9 @@ template <int DIM, int R, bool ISEN, bool BINS>
 cudaError_t sweep_one(const AmrLaunch& L, const int* list, int n, const float4* u1, const float4* u2, float4* o1,
                       float4* o2, const DevClock* clks, cudaStream_t s, int per_sm) {
   auto k = amrk::amr_sweep<DIM, R, ISEN, BINS>;
-  // (set once per instantiation; an attribute call is not a stream operation, so a first call
-  // inside a stream capture is fine)
-  static const cudaError_t attr = [&] {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)amrk::SWEEP_SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-    return e;
-  }();
-  if (attr != cudaSuccess) return attr;
+  static LaunchAttr attr;
+  const cudaError_t e = attr.set((const void*)k, amrk::SWEEP_SMEM, true);
+  if (e != cudaSuccess) return e;
   k<<<grid_for(n, per_sm), amrk::SNT, amrk::SWEEP_SMEM, s>>>(L.gp, L.bt, list, n, u1, u2, L.w1, L.w2, o1, o2, clks, L.fbuf,
                                                              L.err, L.bins, L.fbase, L.p1, L.p2);
   return cudaGetLastError();

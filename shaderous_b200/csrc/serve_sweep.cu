@@ -19,6 +19,7 @@
 #include <cstdint>
 
 #include "amr_device.cuh"
+#include "launch_attr.h"
 #include "sweep_math.cuh"
 #include "tma.cuh"
 
@@ -354,15 +355,9 @@ template <int DIM, int R, bool ISEN>
 cudaError_t launch(const AmrLaunch& L, const int* list, int n, int planes, const float4* u1, const float4* u2, float4* o1,
                    float4* o2, const DevClock* clks, cudaStream_t s) {
   auto k = grid_sweep<DIM, R, ISEN>;
-  // (set once per instantiation; an attribute call is not a stream operation, so a first call
-  // inside a stream capture is fine)
-  static const cudaError_t attr = [&] {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-    return e;
-  }();
-  if (attr != cudaSuccess) return attr;
+  static LaunchAttr attr;
+  const cudaError_t e = attr.set((const void*)k, SMEM, true);
+  if (e != cudaSuccess) return e;
   k<<<grid_for(n * (DIM == 3 ? BS / planes : 1), 4), SNT, SMEM, s>>>(L.gp, L.bt, list, n, planes, u1, u2, L.w1, L.w2, o1, o2,
                                                                     clks, L.err);
   return cudaGetLastError();

@@ -45,6 +45,7 @@
 
 #include "hydro_math.cuh"
 #include "diag_ext.cuh"
+#include "launch_attr.h"
 #include "sweep.h"
 #include "sweep_device.cuh"
 #include "sweep_math.cuh"
@@ -731,17 +732,9 @@ template <int DIM, int RECON, bool ISEN>
 static cudaError_t launch_sweep_t(const KParams& P, const float4* u1, const float4* u2, float4* o1, float4* o2,
                                   const ClockArgs& K, int tz, const SweepMaps* maps, int* err, cudaStream_t s) {
   using G = Geo<DIM, RECON>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(sweep_kernel<DIM, RECON, ISEN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)G::SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    // all of the unified L1/shared storage as shared memory, so that two CTAs fit per SM
-    e = cudaFuncSetAttribute(sweep_kernel<DIM, RECON, ISEN>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static LaunchAttr attr;
+  const cudaError_t e = attr.set((const void*)sweep_kernel<DIM, RECON, ISEN>, G::SMEM_BYTES, true);
+  if (e != cudaSuccess) return e;
   dim3 grid((P.n[0] + G::TX - 1) / G::TX, DIM >= 2 ? (P.n[1] + G::TY - 1) / G::TY : 1,
             DIM == 3 ? (P.n[2] + tz - 1) / tz : 1);
   static const CUtensorMap none{};
