@@ -508,7 +508,7 @@ const char* shz_version(void);
 typedef struct shz_tune_entry {
   int32_t kernel, ndim, recon, isentropic, size_class;  /* the key; size class = floor(log2 units) */
   int32_t variant, per_sm, tz;                          /* the choice (0: the kernel's default) */
-  int32_t candidates;                                   /* shapes timed */
+  int32_t candidates;                                   /* shapes compared */
   float ms, default_ms;                                 /* mean time of the choice and of the default */
 } shz_tune_entry;
 /* Turn the tuner on (default) or off (every launch takes the default shape). Process-wide. */

@@ -244,9 +244,11 @@ void step_taken(shz_sim* s) {
   s->slot = (s->slot + 1) % 3;
 }
 
-// One step whose sweep is run once per candidate for the deepest march (z planes in 3D, y rows in 2D),
-// each at the depth fitted within it, timed, the fastest kept. The sweep reads one parity, clock copy and rate slot and writes others, so the
-// step's result is that of a single launch. A clock held at its stop time is not tuned on (the
+// One step whose sweep is run once per depth that a candidate for the deepest march (z planes in 3D, y
+// rows in 2D) comes to on this grid, timed, the fastest kept. Candidates that come to one depth are one
+// launch: it is timed once and stands for the largest of them, since other grids of the size class are
+// bounded by what is kept. The sweep reads one parity, clock copy and rate slot and writes others, so
+// the step's result is that of a single launch. A clock held at its stop time is not tuned on (the
 // sweep would only copy the state).
 int tuned_step(shz_sim* s) {
   auto launch = [&](const shz::tune::Choice& c) { return launch_step(s, fit_depth(s, c.tz)); };
@@ -272,9 +274,10 @@ int tuned_step(shz_sim* s) {
         cands.push_back(c);
       }
     }
-    const int reps = 2;
+    const int reps = 2, shapes = (int)cands.size();
+    cands = shz::tune::distinct(cands, [&](int most) { return fit_depth(s, most); });
     shz::tune::Choice best;
-    CUDA_OR_FAIL(s, shz::tune::choose(sweep_key(s), cands, launch, s->stream, reps, &best));
+    CUDA_OR_FAIL(s, shz::tune::choose(sweep_key(s), cands, launch, s->stream, reps, &best, shapes));
     s->launches += (long long)cands.size() * (1 + reps);
   }
   step_taken(s);

@@ -78,7 +78,8 @@ bool needs(const Key& k) {
 }
 
 cudaError_t choose(const Key& k, const std::vector<Choice>& candidates,
-                   const std::function<cudaError_t(const Choice&)>& launch, cudaStream_t s, int reps, Choice* out) {
+                   const std::function<cudaError_t(const Choice&)>& launch, cudaStream_t s, int reps, Choice* out,
+                   int shapes) {
   if (candidates.empty()) return cudaErrorInvalidValue;
   cudaEvent_t e0, e1;
   cudaError_t e = cudaEventCreate(&e0);
@@ -107,7 +108,7 @@ cudaError_t choose(const Key& k, const std::vector<Choice>& candidates,
   en.choice = candidates[best];
   en.ms = ms[best];
   en.default_ms = ms[0];
-  en.candidates = (int)candidates.size();
+  en.candidates = shapes > 0 ? shapes : (int)candidates.size();
   {
     std::lock_guard<std::mutex> lk(g_mu);
     g_table[k] = en;

@@ -40,7 +40,7 @@ struct Entry {
   Choice choice;
   float ms = 0.f;          // the chosen candidate's mean time
   float default_ms = 0.f;  // the default candidate's
-  int candidates = 0;
+  int candidates = 0;      // shapes that were compared
 };
 
 // Process-wide switch (on by default). Off: every launch takes the kernel's default shape.
@@ -64,9 +64,30 @@ bool needs(const Key& k);
 
 // Time each candidate's launch functor on stream s (one warm-up launch, then `reps` timed
 // launches with CUDA events), store the fastest for k and return it; candidates[0] is the
-// default. On a launch error the error is returned and nothing is stored.
+// default. On a launch error the error is returned and nothing is stored. shapes: the candidates that
+// the list stands for, where distinct() shortened it (0: the list's own length).
 cudaError_t choose(const Key& k, const std::vector<Choice>& candidates,
-                   const std::function<cudaError_t(const Choice&)>& launch, cudaStream_t s, int reps, Choice* out);
+                   const std::function<cudaError_t(const Choice&)>& launch, cudaStream_t s, int reps, Choice* out,
+                   int shapes = 0);
+
+// Bounds on a depth, one for each depth they come to (depth_of a bound): the largest, at the place of the
+// first that comes to it. Equal launches would be told apart by the noise of their timings.
+inline std::vector<Choice> distinct(const std::vector<Choice>& bounds, const std::function<int(int)>& depth_of) {
+  std::vector<Choice> out;
+  std::vector<int> depths;
+  for (const Choice& c : bounds) {
+    const int d = depth_of(c.tz);
+    size_t i = 0;
+    while (i < depths.size() && depths[i] != d) i++;
+    if (i == depths.size()) {
+      depths.push_back(d);
+      out.push_back(c);
+    } else if (c.tz > out[i].tz) {
+      out[i] = c;
+    }
+  }
+  return out;
+}
 
 std::vector<Entry> entries();
 
