@@ -500,7 +500,8 @@ const char* shz_version(void);
  *     pass for the blocks' own cells and same-level ghosts, then the ghosts beyond a level
  *     change over only the blocks that have them; 5, 6: the split form with its two passes side
  *     by side on a second stream; per_sm = CTAs of the work-list grid per SM;
- *   2 AMR fused sweep: per_sm;
+ *   2 AMR fused sweep: per_sm (served grids have a sweep of their own, whose grid is not tuned; a pin
+ *     holds there too);
  *   3 AMR fine-flux pass: per_sm;
  *   4 the per-block-timestep substeps' assemble: variant 1 one pass, 3 the split form (its
  *     second pass over every block of the substep's list); per_sm.

@@ -352,14 +352,14 @@ __global__ void __maxnreg__(96)
 }
 
 template <int DIM, int R, bool ISEN>
-cudaError_t launch(const AmrLaunch& L, const int* list, int n, int planes, const float4* u1, const float4* u2, float4* o1,
-                   float4* o2, const DevClock* clks, cudaStream_t s) {
+cudaError_t launch(const AmrLaunch& L, const int* list, int n, int planes, int per_sm, const float4* u1, const float4* u2,
+                   float4* o1, float4* o2, const DevClock* clks, cudaStream_t s) {
   auto k = grid_sweep<DIM, R, ISEN>;
   static LaunchAttr attr;
   const cudaError_t e = attr.set((const void*)k, SMEM, true);
   if (e != cudaSuccess) return e;
-  k<<<grid_for(n * (DIM == 3 ? BS / planes : 1), 4), SNT, SMEM, s>>>(L.gp, L.bt, list, n, planes, u1, u2, L.w1, L.w2, o1, o2,
-                                                                    clks, L.err);
+  k<<<grid_for(n * (DIM == 3 ? BS / planes : 1), per_sm), SNT, SMEM, s>>>(L.gp, L.bt, list, n, planes, u1, u2, L.w1, L.w2,
+                                                                         o1, o2, clks, L.err);
   return cudaGetLastError();
 }
 
@@ -386,12 +386,15 @@ cudaError_t launch_grid_sweep(const AmrLaunch& L, const int* list, int n, const 
                               float4* o2, const DevClock* clks, cudaStream_t s, int planes) {
   if (n <= 0) return cudaSuccess;
   if (planes <= 0) planes = grid_sweep_planes(n);
+  // (the grid is not timed here, the split decides more than it; a pinned block sweep's holds here too)
+  tune::Choice c;
+  const int per_sm = tune::pinned(tune::K_AMR_SWEEP, &c) && c.per_sm > 0 ? c.per_sm : 4;
   if (L.ndim == 3) {
-    if (L.isen) { SHZ_RECON_SWITCH(L.recon, true, return (gridsw::launch<3, R, true>(L, list, n, planes, u1, u2, o1, o2, clks, s))) }
-    else { SHZ_RECON_SWITCH(L.recon, false, return (gridsw::launch<3, R, false>(L, list, n, planes, u1, u2, o1, o2, clks, s))) }
+    if (L.isen) { SHZ_RECON_SWITCH(L.recon, true, return (gridsw::launch<3, R, true>(L, list, n, planes, per_sm, u1, u2, o1, o2, clks, s))) }
+    else { SHZ_RECON_SWITCH(L.recon, false, return (gridsw::launch<3, R, false>(L, list, n, planes, per_sm, u1, u2, o1, o2, clks, s))) }
   } else {
-    if (L.isen) { SHZ_RECON_SWITCH(L.recon, true, return (gridsw::launch<2, R, true>(L, list, n, planes, u1, u2, o1, o2, clks, s))) }
-    else { SHZ_RECON_SWITCH(L.recon, false, return (gridsw::launch<2, R, false>(L, list, n, planes, u1, u2, o1, o2, clks, s))) }
+    if (L.isen) { SHZ_RECON_SWITCH(L.recon, true, return (gridsw::launch<2, R, true>(L, list, n, planes, per_sm, u1, u2, o1, o2, clks, s))) }
+    else { SHZ_RECON_SWITCH(L.recon, false, return (gridsw::launch<2, R, false>(L, list, n, planes, per_sm, u1, u2, o1, o2, clks, s))) }
   }
   return cudaSuccess;
 }

@@ -18,7 +18,7 @@ namespace tune {
 enum Kernel : int {
   K_UNIFORM_SWEEP = 0,  // tz: the most planes a CTA marches along z (3D); 2D (>= 512 a side): rows along y
   K_AMR_ASSEMBLE = 1,   // variant: register budget (CTAs per SM the compiler plans for); per_sm: grid
-  K_AMR_SWEEP = 2,      // per_sm: grid
+  K_AMR_SWEEP = 2,      // per_sm: grid (served grids' sweep is not timed, but a pin holds there too)
   K_AMR_FINE_FLUX = 3,  // per_sm: grid
   K_AMR_ASSEMBLE_BINS = 4,  // the per-block-timestep substeps' assemble: variant 1 one pass, 3 split
   K_COUNT = 5

@@ -4,7 +4,7 @@ the GPU (whole blocks) ends in the same state, bit for bit; and in the plain ste
 import numpy as np
 import pytest
 
-from shaderous_b200 import Config, Problem, Sim
+from shaderous_b200 import Config, Problem, Sim, tune
 from shaderous_b200.serve import Request, Server, ServerConfig
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +42,21 @@ def test_split_blocks_give_the_whole_blocks_bits(recon, isen, bc, prob):
     # nine steps of the same arithmetic in two kernels: a few float32 roundings of the largest values
     for got, ref in zip(alone[1], (p1, p2)):
         assert np.abs(got - ref).max() <= 9 * 8 * 2.0 ** -24 * np.abs(ref).max()
+
+
+def test_a_pinned_grid_gives_the_same_bits():
+    """The block sweep's pinned CTAs per SM hold for served grids too. At one an SM a CTA takes several
+    blocks, one after another, in 2D and in 3D."""
+    hyd = Config(recon="koren", isentropic=True, cfl=0.4, p_floor=1e-12)
+    reqs = [Request(ndim=3, n=112, steps=5, problem=BLAST, gamma=1.4, bc=2),
+            Request(ndim=2, n=400, steps=7, problem=BLAST, gamma=1.4, bc=1),
+            Request(ndim=3, n=16, steps=3, problem=BLAST, gamma=1.4, bc=1)]  # held while the others run on
+    ref = _served(hyd, reqs)
+    for per_sm in (1, 2):
+        tune.pin("amr_sweep", 0, per_sm)
+        try:
+            got = _served(hyd, reqs)
+        finally:
+            tune.pin("amr_sweep", None)
+        for (a1, a2), (b1, b2) in zip(ref, got):
+            assert np.array_equal(a1, b1) and np.array_equal(a2, b2), per_sm
