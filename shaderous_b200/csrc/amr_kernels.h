@@ -100,11 +100,10 @@ cudaError_t amr_launch_fine_flux(const AmrLaunch& L, const int* flist, int nf, c
 cudaError_t amr_launch_sweep(const AmrLaunch& L, const int* list, int n, const float4* u1, const float4* u2, float4* o1,
                              float4* o2, const DevClock* clks, cudaStream_t s, const tune::Choice* c = nullptr);
 // The same for the blocks of uniform grids at level 0 (serve_sweep.cu), where no ghost and no face lies at
-// a level change: the uniform sweeps' arithmetic, and `planes` planes of a block a CTA (3D; 16, 8, 4
-// or 2; 0: as many as fill the SMs best). Every split gives the same bits.
+// a level change: the uniform sweeps' arithmetic, and in 3D 16, 8, 4 or 2 planes of a block a CTA, which
+// fill the SMs best. Every split gives the same bits.
 cudaError_t launch_grid_sweep(const AmrLaunch& L, const int* list, int n, const float4* u1, const float4* u2, float4* o1,
-                              float4* o2, const DevClock* clks, cudaStream_t s, int planes = 0);
-int grid_sweep_planes(int n);
+                              float4* o2, const DevClock* clks, cudaStream_t s);
 // Per-block timesteps, fused form: the leaves in list half way through their step beside a faster
 // neighbour take that neighbour's second-step fluxes from fbuf, in place (amr/update.wgsl deposit).
 cudaError_t amr_launch_deposit(const AmrLaunch& L, const int* list, int n, float4* u1, float4* u2, const DevClock* clks,

@@ -363,16 +363,14 @@ cudaError_t launch(const AmrLaunch& L, const int* list, int n, int planes, int p
   return cudaGetLastError();
 }
 
-}  // namespace gridsw
-
 // The planes of a block a CTA marches: the split whose parts fill the SMs best. A part of p planes
 // takes about p + 4 plane times (two planes predicted only, the first copies); two parts run side by
 // side on an SM, and one alone takes 0.65 of its time beside another.
-int grid_sweep_planes(int n) {
+int planes_of(int n) {
   double best = 0.0;
-  int planes = amrk::BS;
-  for (int p = amrk::BS; p >= 2; p /= 2) {
-    const int per = (int)(((long long)n * (amrk::BS / p) + 147) / 148);
+  int planes = BS;
+  for (int p = BS; p >= 2; p /= 2) {
+    const int per = (int)(((long long)n * (BS / p) + 147) / 148);
     const double cost = (p + 4) * (per / 2 + 0.65 * (per % 2));
     if (best == 0.0 || cost < best) {
       best = cost;
@@ -382,10 +380,12 @@ int grid_sweep_planes(int n) {
   return planes;
 }
 
+}  // namespace gridsw
+
 cudaError_t launch_grid_sweep(const AmrLaunch& L, const int* list, int n, const float4* u1, const float4* u2, float4* o1,
-                              float4* o2, const DevClock* clks, cudaStream_t s, int planes) {
+                              float4* o2, const DevClock* clks, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  if (planes <= 0) planes = grid_sweep_planes(n);
+  const int planes = gridsw::planes_of(n);
   // (the grid is not timed here, the split decides more than it; a pinned block sweep's holds here too)
   tune::Choice c;
   const int per_sm = tune::pinned(tune::K_AMR_SWEEP, &c) && c.per_sm > 0 ? c.per_sm : 4;

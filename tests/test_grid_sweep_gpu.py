@@ -44,6 +44,35 @@ def test_split_blocks_give_the_whole_blocks_bits(recon, isen, bc, prob):
         assert np.abs(got - ref).max() <= 9 * 8 * 2.0 ** -24 * np.abs(ref).max()
 
 
+# Requests beside one of a single 3D block, the blocks of the whole batch, and the planes of a block a CTA
+# marches there: of 16, 8, 4 and 2 the p with the least (p + 4) (c / 2 + 0.65 (c mod 2)), c the CTAs of the
+# fullest of 148 SMs (two run side by side on one).
+BATCHES = [((), 1, 2), ((32, 32), 17, 2), ((32, 32, 32), 25, 4), ((64,), 65, 8), ((96,), 217, 8), ((96, 32), 225, 16),
+           ((112, 48), 371, 16)]
+
+
+def _planes(n):
+    def cost(p):
+        c = -(-n * (16 // p) // 148)
+        return (p + 4) * (c // 2 + 0.65 * (c % 2))
+
+    return min((16, 8, 4, 2), key=cost)
+
+
+@pytest.mark.parametrize("bc", [0, 1, 2])
+def test_every_split_gives_the_same_bits(bc):
+    hyd = Config(recon="koren", isentropic=True, cfl=0.4, p_floor=1e-12)
+    one = Request(ndim=3, n=16, steps=8, problem=BLAST, gamma=1.4, bc=bc)
+    first, splits = None, set()
+    for beside, blocks, planes in BATCHES:
+        assert 1 + sum((n // 16) ** 3 for n in beside) == blocks and _planes(blocks) == planes
+        splits.add(planes)
+        got = _served(hyd, [one] + [Request(ndim=3, n=n, steps=8, problem=BLAST, gamma=1.4, bc=bc) for n in beside])[0]
+        first = first or got
+        assert np.array_equal(first[0], got[0]) and np.array_equal(first[1], got[1]), beside
+    assert splits == {2, 4, 8, 16}
+
+
 def test_a_pinned_grid_gives_the_same_bits():
     """The block sweep's pinned CTAs per SM hold for served grids too. At one an SM a CTA takes several
     blocks, one after another, in 2D and in 3D."""
