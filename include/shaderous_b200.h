@@ -229,7 +229,7 @@ int shz_halo_depth(const shz_sim* sim, int32_t* planes);
  * in u2 (depth x nx x ny float4, x fastest). */
 int shz_halo_device(shz_sim* sim, int32_t side, void** inner_u1, void** inner_u2, void** ghost_u1, void** ghost_u2,
                     size_t* bytes);
-/* The device word the next step's clock reads its rate from (uint32 bits of the largest
+/* The device word the next step takes its rate from (uint32 bits of the largest
  * rate / dx over this slab after its last step, or after shz_set_state / shz_reset_problem). */
 int shz_rate_device(shz_sim* sim, void** rate);
 /* The handle's CUDA stream (a cudaStream_t), to order the caller's transfers with the steps. */
@@ -240,7 +240,7 @@ int shz_stream(shz_sim* sim, void** stream);
  * total device time of the steps, and the summed time of the sweep kernels alone. Blocking. */
 typedef struct shz_profile_result {
   int32_t steps;
-  double total_ms;   /* first clock kernel's start to last sweep's end */
+  double total_ms;   /* first sweep's start to last sweep's end, the events between them included */
   double sweep_ms;   /* sum over the n sweeps of each sweep's own duration */
   int64_t launches;  /* kernels launched for the n steps */
 } shz_profile_result;
@@ -491,8 +491,9 @@ const char* shz_version(void);
  * fastest in a process-wide table, and uses it from then on (also in captured CUDA graphs).
  * Candidates differ only in launch shape, never in arithmetic: the state is the same whichever
  * wins. Kernels and their knobs:
- *   0 uniform sweep: tz = planes a CTA marches along z (3D); in 2D grids of at least 512 cells
- *     a side, the rows a CTA marches along y (smaller 2D grids take a tile form, 16 x 12 cells
+ *   0 uniform sweep: tz = the most planes a CTA marches along z (3D); in 2D grids of at least 512
+ *     cells a side, the most rows a CTA marches along y (the depth that runs is fitted to the grid
+ *     within it, or is the pinned one; smaller 2D grids take a tile form, 16 x 12 cells
  *     with a ring of halo cells, untuned; the two forms agree to rounding, each depth of one form
  *     gives the same bits);
  *   1 AMR assemble: variant = register budget (0: 1, 1: 2, 2: 3 CTAs per SM) of the one-pass

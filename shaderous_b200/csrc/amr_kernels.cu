@@ -918,7 +918,7 @@ cudaError_t amr_launch_gather_grid(int ndim, const int* list, int nr, const floa
   return cudaGetLastError();
 }
 
-// The clocks of many grids at once, one thread each: as step_clock (sweep.cu), reading grid
+// The clocks of many grids at once, one thread each: as step_clock (sweep_device.cuh), reading grid
 // g's rate from rates[2 g + rslot] and clearing the other slot for the next step; a grid that
 // has taken max_steps steps holds.
 __global__ void clock_multi_kernel(DevClock* __restrict__ clks, unsigned* __restrict__ rates, int rslot, int ngrids,

@@ -1,7 +1,7 @@
-// The block passes' arithmetic of one cell and one face (the adaptive grid and the served blocks:
-// amr_*.cu): limiters, the density along the adiabat, the Hancock step, face states, the HLLC/HLL
-// flux and the update. The uniform sweeps have the same scheme in sweep_math.cuh, in a form of
-// fewer instructions that rounds differently in places. This form keeps its rounding: refinement is
+// The adaptive grid's arithmetic of one cell and one face (amr_*.cu): limiters, the density along the
+// adiabat, the Hancock step, face states, the HLLC/HLL flux and the update. The sweeps of uniform grids
+// and of served blocks have the same scheme in sweep_math.cuh, in a form of fewer instructions that
+// rounds differently in places. This form keeps its rounding: refinement is
 // decided by thresholds on what it computes, so that another rounding gives another mesh (on a mesh
 // of 6,000 blocks, one block's decision within a dozen checks).
 #pragma once

@@ -199,7 +199,8 @@ int refresh_rate(shz_sim* s) {
 // is fixed by the grid's size, not by timing: the two forms are different kernels, which agree to
 // rounding (the compiler may contract a multiply and an add differently in each), while every
 // depth of one form is the same kernel and gives the same bits. 2D grids of at least 512 cells a
-// side march along y; smaller ones take the tile form. The tuner's choice (64 planes or 16 rows
+// side march along y; smaller ones take the tile form (a pin picks the form too: a depth the march, 0 the
+// tiles, on grids of any size). The tuner's choice (64 planes or 16 rows
 // untuned) is the deepest march: the keys are size classes, which grids of many shapes share, and
 // within it the depth that runs is fitted to this grid's own columns (sweep_fit_depth). A pinned
 // depth runs as it is.

@@ -1,4 +1,4 @@
-// The uniform-grid hydro step as one fused kernel per step, plus its clock, rate and
+// The uniform-grid hydro step as one fused kernel per step, its clock included, plus the rate and
 // diagnostics kernels.
 //
 // One step of the reference (src/sim.ts:3187-3328 encodeSteps) is four passes: rates
@@ -13,9 +13,10 @@
 // maximum (warp shuffles, then one atomicMax per CTA on the float's bits).
 //
 // Small grids are bound by the chain of launches. With the clock a kernel of its own, a step took
-// 10.7 us on a tube of 512 cells and 13.4 us on a 64^2 grid (runs of 64 steps); with the clock in the
-// sweep, and the next step's launch overlapped with this one's work (programmatic dependent launch:
-// step_clock waits for the step before), 6.5 and 8.6 us. Large grids take the same time either way.
+// 10.7 us on a tube of 512 cells and 13.4 us on a 64^2 grid (runs of 64 steps, their seven looks at the
+// clock included); with the clock in the sweep, and the next step's launch overlapped with this one's
+// work (programmatic dependent launch: step_clock waits for the step before), 6.5 and 8.6 us; with the
+// looks that shz_run now takes, 3.3 and 5.2 us. Large grids take the same time either way.
 //
 // Decomposition: a CTA owns a TX x TY column of cells and marches it along z through tz planes
 // (2.5D). Its threads are the column's TX x TY cells and one a halo cell across each of its four sides

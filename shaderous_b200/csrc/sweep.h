@@ -26,9 +26,9 @@ bool encode_sweep_maps(SweepMaps* m, const float4* base1, const float4* base2, i
                        int recon);
 
 // tz: planes a CTA marches along z (3D; 0 for the default); in 2D, rows a CTA marches along y (the
-// row form), or 0 for the tile form. Every tz gives the same state, with or without maps (the
-// staging path and the per-cell loads give the same primitives). err: the kernel's error word (a
-// bounded wait for a copy that ran out), or null.
+// row form), or 0 for the tile form. Every depth of one form gives the same state, with or without
+// maps (the staging path and the per-cell loads give the same primitives); the two 2D forms agree to
+// rounding. err: the kernel's error word (a bounded wait for a copy that ran out), or null.
 constexpr int SWEEP_TZ_DEFAULT = 64;
 // A step's clock and rate words: `in` and `rate` as the last step left them, `out` the other copy of the
 // clock, `rate_out` the (empty) slot this step folds its rates into, `rate_next` the third slot,

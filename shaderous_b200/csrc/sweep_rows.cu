@@ -75,8 +75,8 @@ __device__ __forceinline__ void read_row(const float* __restrict__ sWr, int wx, 
 }
 
 template <int RECON, bool ISEN>
-// (5 CTAs of 4 warps per SM: 96 registers a thread; at 128 and 4 CTAs, or at 80 and 6 with spills,
-// the Kelvin-Helmholtz march ran 4-8 % slower)
+// (5 CTAs of 4 warps per SM: 96 registers a thread, at which only PPM spills, 42 bytes; at 128 and 4
+// CTAs, or at 80 and 6 with more spills, the Kelvin-Helmholtz march ran 4-8 % slower)
 __global__ void __launch_bounds__(RowGeo<RECON>::NT, 5)
     sweep_rows_kernel(const KParams P, const float4* __restrict__ u1, const float4* __restrict__ u2,
                       float4* __restrict__ o1, float4* __restrict__ o2, const ClockArgs K, int rows) {

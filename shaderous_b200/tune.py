@@ -3,7 +3,8 @@
 The first time a handle runs a tunable kernel for a (kernel, ndim, reconstruction, isentropic,
 size class) key, the library times every candidate launch shape in place, inside one real step,
 and keeps the fastest for the rest of the process. Candidates differ only in launch shape, so the
-state is the same whichever wins.
+state is the same whichever wins. (A pinned depth in 2D also picks one of two kernels, which agree to
+rounding: see :func:`pin`.)
 """
 from __future__ import annotations
 
@@ -29,7 +30,8 @@ def pin(kernel: str, variant: int | None, per_sm: int = 0) -> None:
     unpins. AMR kernels ("amr_assemble", "amr_sweep", "amr_fine_flux", "amr_assemble_bins"): a
     variant and CTAs per SM. The sweep of served grids is not tuned; "amr_sweep" pins its CTAs per SM
     too. "uniform_sweep": variant 0 and ``per_sm`` = its depth (z planes a
-    CTA marches in 3D; in 2D the rows it marches along y, 0 for the tile form)."""
+    CTA marches in 3D; in 2D the rows it marches along y, 0 for the tile form, whatever the grid's size;
+    unpinned, the form follows the size and the depth is fitted to the grid within the tuned one)."""
     k = {v: n for n, v in KERNELS.items()}[kernel]
     rc = _abi.load().shz_tune_pin(k, -1 if variant is None else int(variant), int(per_sm))
     if rc != 0:
